@@ -106,10 +106,11 @@ enum gpr_src { SRC_X = 0, SRC_C = 1, SRC_ONE = 2, SRC_POP = 3, SRC_X2 = 4, SRC_X
 
 /* Counters the MH kernel accumulates (gpr_get_stats). */
 enum gpr_stat {
-    GPR_STAT_EVALS = 0,        /* likelihood evaluations (one per proposal + one per chain) */
-    GPR_STAT_EVAL_NODES,       /* sum over evaluations of the program's node count          */
-    GPR_STAT_EVAL_POINTS,      /* data points actually evaluated (early exit on invalid)   */
-    GPR_STAT_EVAL_NODE_POINTS, /* sum over evaluations of (node count + 4) * points        */
+    GPR_STAT_EVALS = 0,        /* likelihoods scored (one per proposal + one per chain)     */
+    GPR_STAT_EVAL_NODES,       /* sum over them of the program's node count                 */
+    GPR_STAT_EVAL_POINTS,      /* data points actually evaluated (none for a proposal that
+                                * keeps the current values; early exit on invalid)          */
+    GPR_STAT_EVAL_NODE_POINTS, /* sum over evaluated points of node count + 4               */
     GPR_STAT_STRUCT_PROPOSED,
     GPR_STAT_STRUCT_ACCEPTED,
     GPR_STAT_CONST_PROPOSED,

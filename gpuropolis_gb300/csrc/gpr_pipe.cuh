@@ -39,8 +39,11 @@ struct PipeSlot {
     df prior, cs;                 /* the proposal in flight: prior, Cauchy sum                           */
     df fw, bw;                    /* forward/backward terms (main.cu:702,723,761-775)                    */
     int chain;                    /* >= p.N: no chain in this slot                                       */
-    int cur, ccur, pbuf, cbuf;    /* ops/program and constants buffers: current, proposal                */
+    int cur, ccur, gcur;          /* ops, constants and program buffers of the current state             */
+    int pbuf, cbuf, gbuf;         /* ... and of the proposal                                             */
     int ninstr, count, cur_ninstr, cur_count;
+    int same;                     /* the proposal's values are the current state's: S is cur_S           */
+    int reads, cur_reads;         /* the program reads constants: proposal, current                      */
     float len, cur_len;
     uint32_t rs, rblk, rw0, rw1, rw2, rw3;   /* the chain's random stream                           */
     float rw_sd, log_sd;          /* random-walk scale and its adaptation state                         */
@@ -212,13 +215,15 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                 const int step = (h - g) / 2 - 1;   /* the step proposed now: -1 the loaded state */
                 const WarpSmem wg = carve_pipe<K>(mybase, PL, p.max_instr, p.levels, g);
                 int publish = -1;
-                int pbuf = 0, cbuf = 0, count = 0;
+                int gbuf = 0, cbuf = 0, count = 0;
                 if (chain < p.N) {
                     /* the chain's state, into registers */
                     df cur_prior = SS.cur_prior, cur_S = SS.cur_S, cur_cs = SS.cur_cs;
                     df prior = SS.prior, cs = SS.cs, fw = SS.fw, bw = SS.bw;
-                    int cur = SS.cur, ccur = SS.ccur;
-                    pbuf = SS.pbuf; cbuf = SS.cbuf;
+                    int cur = SS.cur, ccur = SS.ccur, gcur = SS.gcur;
+                    int pbuf = SS.pbuf;
+                    cbuf = SS.cbuf; gbuf = SS.gbuf;
+                    bool same = SS.same != 0, reads = SS.reads != 0, cur_reads = SS.cur_reads != 0;
                     int ninstr = SS.ninstr, cur_ninstr = SS.cur_ninstr, cur_count = SS.cur_count;
                     count = SS.count;
                     float len = SS.len, cur_len = SS.cur_len;
@@ -232,7 +237,9 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                         /* the accept rule for the proposal of step - 1 (the loaded state when step == 0) */
                         const bool init = step == 0;
                         df S;
-                        if (s_bad[g][warp]) {
+                        if (same) {
+                            S = cur_S;
+                        } else if (s_bad[g][warp]) {
                             S = lik_invalid();
                         } else {
                             const float* pr = part_row(g, warp);
@@ -253,7 +260,7 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                         }
                         ST_ADD(GPR_STAT_EVALS, 1); ST_ADD(GPR_STAT_EVAL_NODES, count);
                         if (accept) {
-                            cur = pbuf; ccur = cbuf;
+                            cur = pbuf; ccur = cbuf; gcur = gbuf; cur_reads = reads;
                             cur_len = len; cur_count = count; cur_ninstr = ninstr; cur_cs = cs;
                             cur_prior = prior; cur_S = S;
                         }
@@ -270,7 +277,8 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                         }
                         __syncwarp();
                         r = rng_start<RNG>(p.seed, chain);
-                        cur = ccur = pbuf = cbuf = 0;
+                        cur = ccur = gcur = pbuf = cbuf = gbuf = 0;
+                        reads = cur_reads = false;
                         cur_ninstr = cur_count = 0; cur_len = 0.0f;
                         cur_prior = cur_S = cur_cs = df_make(0.0f, 0.0f);
                         fw = bw = df_make(0.0f, 0.0f);
@@ -283,29 +291,36 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                         const bool init = step < 0;
                         structural = !init && p.struct_every > 0 && (step % p.struct_every == 0);
                         bool need_compile = init;
+                        same = false;   /* as in mh_block_kernel: no evaluation for unchanged values */
                         if (structural) {
                             /* ---- structure move (main.cu:699-742) ---- */
                             fw = df_make(-p.logcount[cur_count], 0.0f);
                             const bool cur_invalid = !(isfinite(cur_prior.hi) && isfinite(cur_S.hi));
-                            structure_move<RNG>(r, wg.ops[cur], wg.ops[cur ^ 1], cur_invalid, p, s_lj[lane], lane);
-                            pbuf = cur ^ 1; cbuf = ccur;
-                            need_compile = true;
+                            need_compile = structure_move<RNG>(r, wg.ops[cur], wg.ops[cur ^ 1], cur_invalid, p,
+                                                               s_lj[lane], lane);
+                            same = !need_compile;
+                            pbuf = cur ^ 1; cbuf = ccur; gbuf = same ? gcur : gcur ^ 1;
+                            len = cur_len; count = cur_count; ninstr = cur_ninstr; reads = cur_reads;
                             GPR_PH(GPR_PH_STRUCT);
                         } else if (!init) {
                             /* ---- constant move (main.cu:743-806) ---- */
                             df fws, bws;
                             constant_move<RNG>(r, wg, wg.Cs[ccur], wg.Cs[ccur ^ 1], fws, bws, p, s_lj[lane], lane, rw_sd);
                             if (p.const_mode == 0) { fw = df_add(fw, fws); bw = df_add(bw, bws); }
-                            pbuf = cur; cbuf = ccur ^ 1;
-                            len = cur_len; count = cur_count; ninstr = cur_ninstr;
+                            pbuf = cur; cbuf = ccur ^ 1; gbuf = gcur;
+                            len = cur_len; count = cur_count; ninstr = cur_ninstr; reads = cur_reads;
+                            same = !reads;
                             GPR_PH(GPR_PH_CONST);
                         }
                         __syncwarp();
                         if (need_compile) {
-                            const CompileOut co = compile_parallel<NV>(wg.ops[pbuf], PL, wg.prog[pbuf],
+                            const CompileOut co = compile_parallel<NV>(wg.ops[pbuf], PL, wg.prog[gbuf],
                                                                    compile_scratch(wg.stk, PL), lane);
                             len = co.length; count = co.count; ninstr = co.ninstr;
                             __syncwarp();
+                            bool rd = false;
+                            for (int i = lane; i < ninstr; i += 32) rd = rd || reads_constant(wg.prog[gbuf][i]);
+                            reads = __any_sync(FULLMASK, rd);
                             GPR_PH(GPR_PH_COMPILE);
                         }
                         if (structural) {
@@ -316,7 +331,7 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                             GPR_PH(GPR_PH_CAUCHY);
                         }
                         prior = prior_u(len, cs, p);
-                        publish = ninstr;
+                        publish = same ? -1 : ninstr;
                     } else {
                         /* write back (main.cu:811-812 and the in-place P, C) */
                         for (int i = lane; i < PL; i += 32) {
@@ -335,7 +350,8 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                     if (lane == 0) {
                         SS.cur_prior = cur_prior; SS.cur_S = cur_S; SS.cur_cs = cur_cs;
                         SS.prior = prior; SS.cs = cs; SS.fw = fw; SS.bw = bw;
-                        SS.cur = cur; SS.ccur = ccur; SS.pbuf = pbuf; SS.cbuf = cbuf;
+                        SS.cur = cur; SS.ccur = ccur; SS.gcur = gcur; SS.pbuf = pbuf; SS.cbuf = cbuf; SS.gbuf = gbuf;
+                        SS.same = same; SS.reads = reads; SS.cur_reads = cur_reads;
                         SS.ninstr = ninstr; SS.count = count; SS.cur_ninstr = cur_ninstr; SS.cur_count = cur_count;
                         SS.len = len; SS.cur_len = cur_len;
                         SS.rs = r.s; SS.rblk = r.blk; SS.rw0 = r.w0; SS.rw1 = r.w1; SS.rw2 = r.w2; SS.rw3 = r.w3;
@@ -348,7 +364,7 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                     s_cost[g][warp] = publish;
                     s_cnt[g][warp] = count;
                     s_bad[g][warp] = 0;
-                    s_pp[g][warp] = wg.prog[pbuf & 1];
+                    s_pp[g][warp] = wg.prog[gbuf & 1];
                     s_pc[g][warp] = wg.Cs[cbuf & 1];
                 }
                 __syncwarp();

@@ -242,9 +242,10 @@ int gpr_layout_lockstep(gpr_handle* h);
 int gpr_layout_pipelined(gpr_handle* h);
 
 /* Counters accumulated by the MH kernel since the last reset (no reference
- * counterpart): [0] likelihood evaluations, [1] sum of evaluated node counts,
- * [2] data points evaluated, [3] sum of (node count + 4) * points (the
- * algorithmic FP32 work), [4]/[5] structure moves proposed/accepted,
+ * counterpart): [0] likelihoods scored (one per proposal and one per chain and
+ * block), [1] sum of their node counts, [2] data points evaluated to score
+ * them (a proposal with the current state's values needs none), [3] sum of
+ * (node count + 4) over those points (the algorithmic FP32 work), [4]/[5] structure moves proposed/accepted,
  * [6]/[7] constant moves proposed/accepted.  Copies min(n, 8) values. */
 int gpr_get_stats(gpr_handle* h, uint64_t* out, int n);
 int gpr_reset_stats(gpr_handle* h);
