@@ -69,7 +69,9 @@ struct gpr_handle {
     unsigned long long* dkeys = nullptr;   /* N posterior keys                   */
     unsigned long long* dsel = nullptr;    /* [0] selected key (per dataset)     */
     int dsel_cap = 0;
-    int* dseli = nullptr;                  /* [0] count, [1] first index         */
+    int* dseli = nullptr;                  /* [0] count                          */
+    gpr::SelectResult* hsel = nullptr;     /* pinned: the selection's result, then room for the first
+                                            * GPR_TOP_STAGE candidate chains     */
     int* dtop = nullptr;                   /* candidate chains, dtop_cap entries */
     int dtop_cap = 0;
     int nd = -1;
@@ -201,6 +203,7 @@ int64_t gpr_launch_count(gpr_handle* h) { return h ? h->launches : 0; }
 static void free_all(gpr_handle* h) {
     cudaFree(h->dP); cudaFree(h->dC); cudaFree(h->dprior); cudaFree(h->dlik);
     cudaFree(h->dlogcount); cudaFree(h->dcounter); cudaFree(h->ddata); cudaFree(h->dstats);
+    cudaFreeHost(h->hsel);
     cudaFree(h->dkeys); cudaFree(h->dsel); cudaFree(h->dseli); cudaFree(h->dtop); cudaFree(h->dscale);
     cudaFree(h->dds); cudaFree(h->dds_ns); cudaFree(h->dds_ns64); cudaFree(h->dpart);
     if (h->graph) cudaGraphExecDestroy(h->graph);
@@ -1309,7 +1312,13 @@ int gpr_run_block_traced(gpr_handle* h, int steps, int random_seed, int trace_n,
 
 /* ---- selection over posteriors (gpr_resample.cu) ---- */
 
+/* Candidate chains copied back together with their number. */
+#define GPR_TOP_STAGE 2048
+
 static int ensure_select(gpr_handle* h) {
+    if (!h->hsel)
+        CUDA_TRY(h, cudaHostAlloc((void**)&h->hsel, sizeof(gpr::SelectResult) + GPR_TOP_STAGE * sizeof(int),
+                                  cudaHostAllocDefault));
     if (!h->dkeys) {
         CUDA_TRY(h, cudaMalloc(&h->dkeys, (size_t)h->N * sizeof(unsigned long long)));
         CUDA_TRY(h, cudaMalloc(&h->dseli, 4 * sizeof(int)));
@@ -1322,19 +1331,6 @@ static int ensure_select(gpr_handle* h) {
         h->dsel_cap = 0;
         CUDA_TRY(h, cudaMalloc(&h->dsel, (size_t)need * sizeof(unsigned long long)));
         h->dsel_cap = need;
-    }
-    return GPR_OK;
-}
-
-/* The posterior at ascending rank `rank` (reference comparator order). */
-static int select_rank(gpr_handle* h, int rank, unsigned long long* key) {
-    int rc = ensure_select(h);
-    if (rc != GPR_OK) return rc;
-    CUDA_TRY(h, gpr::launch_select(h->kp, rank, h->dkeys, h->dsel, h->stream));
-    h->launches += 2;
-    if (key) {
-        CUDA_TRY(h, cudaMemcpyAsync(key, h->dsel, sizeof *key, cudaMemcpyDeviceToHost, h->stream));
-        CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     }
     return GPR_OK;
 }
@@ -1359,22 +1355,24 @@ int gpr_resample_datasets(gpr_handle* h, int mode, double param, uint32_t seed, 
     CUDA_TRY(h, cudaSetDevice(h->device));
     int rc = ensure_select(h);
     if (rc != GPR_OK) return rc;
-    CUDA_TRY(h, gpr::launch_select(h->kp, rank, h->dkeys, h->dsel, h->stream, nseg));
-    h->launches += 2;
-    CUDA_TRY(h, cudaMemsetAsync(h->dseli, 0, sizeof(int), h->stream));
+    CUDA_TRY(h, gpr::launch_select(h->kp, rank, h->dkeys, h->dsel, h->dseli, nseg == 1 ? h->hsel : nullptr,
+                                   h->stream, nseg));
+    h->launches++;
     const gpr::Magic mops1 = magic_for(divisor_for(h->cfg.n_ops - 1));
     const gpr::Magic morder = magic_for(divisor_for(8));
-    CUDA_TRY(h, gpr::launch_redraw(h->kp, h->dsel, nseg > 1 ? seg : 0, mode, param, seed, mops1, morder, h->dseli,
-                                   h->stream));
-    h->launches++;
+    CUDA_TRY(h, gpr::launch_redraw(h->kp, h->dsel, nseg > 1 ? seg : 0, mode, param, seed, mops1, morder,
+                                   (int*)h->dkeys, h->dseli, h->stream));   /* the keys are used up: their memory lists the chains */
+    h->launches += 2;
     if (n_redrawn || cutoffs) {
         std::vector<unsigned long long> keys((size_t)nseg);
-        int cnt = 0;
-        CUDA_TRY(h, cudaMemcpyAsync(keys.data(), h->dsel, (size_t)nseg * sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, h->stream));
-        CUDA_TRY(h, cudaMemcpyAsync(&cnt, h->dseli, sizeof cnt, cudaMemcpyDeviceToHost, h->stream));
+        if (cutoffs && nseg > 1)
+            CUDA_TRY(h, cudaMemcpyAsync(keys.data(), h->dsel, (size_t)nseg * sizeof(unsigned long long),
+                                        cudaMemcpyDeviceToHost, h->stream));
+        if (n_redrawn)
+            CUDA_TRY(h, cudaMemcpyAsync(&h->hsel->count, h->dseli, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
         CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-        if (n_redrawn) *n_redrawn = cnt;
+        if (nseg == 1) keys[0] = h->hsel->key;
+        if (n_redrawn) *n_redrawn = h->hsel->count;
         if (cutoffs)
             for (int d = 0; d < nseg; ++d) cutoffs[d] = gpr_key_value(keys[d]) - (mode == 1 ? param : 0.0);
     }
@@ -1405,9 +1403,9 @@ int gpr_resample_below(gpr_handle* h, double cutoff, uint32_t seed, int chain_of
     CUDA_TRY(h, cudaMemsetAsync(h->dseli, 0, sizeof(int), h->stream));
     const gpr::Magic mops1 = magic_for(divisor_for(h->cfg.n_ops - 1));
     const gpr::Magic morder = magic_for(divisor_for(8));
-    CUDA_TRY(h, gpr::launch_redraw(h->kp, h->dsel, 0, 0, 0.0, seed, mops1, morder, h->dseli, h->stream,
-                                   (uint32_t)chain_offset));
-    h->launches++;
+    CUDA_TRY(h, gpr::launch_redraw(h->kp, h->dsel, 0, 0, 0.0, seed, mops1, morder, (int*)h->dkeys, h->dseli,
+                                   h->stream, (uint32_t)chain_offset));
+    h->launches += 2;
     /* the key's host copy must outlive the asynchronous copy: wait here */
     int cnt = 0;
     CUDA_TRY(h, cudaMemcpyAsync(&cnt, h->dseli, sizeof cnt, cudaMemcpyDeviceToHost, h->stream));
@@ -1423,13 +1421,8 @@ int gpr_top_chains(gpr_handle* h, int k, double margin, int* chains, int capacit
     if (!(margin >= 0.0)) return fail(h, GPR_ERR_ARG, "margin %g is not >= 0", margin);
     if (capacity < 0 || (capacity > 0 && !chains) || !n) return fail(h, GPR_ERR_ARG, "bad output arguments");
     CUDA_TRY(h, cudaSetDevice(h->device));
-    unsigned long long key = 0;
-    int rc = select_rank(h, h->N - k, &key);
+    int rc = ensure_select(h);
     if (rc != GPR_OK) return rc;
-    const double t = gpr_key_value(key);
-    if (threshold) *threshold = t;
-    /* every non-NaN chain when fewer than k are non-NaN */
-    const unsigned long long kmin = key == 0ull ? 1ull : gpr_post_key(t - margin);
     if (capacity > h->dtop_cap) {
         CUDA_TRY(h, cudaStreamSynchronize(h->stream));
         cudaFree(h->dtop);
@@ -1438,18 +1431,26 @@ int gpr_top_chains(gpr_handle* h, int k, double margin, int* chains, int capacit
         CUDA_TRY(h, cudaMalloc(&h->dtop, (size_t)capacity * sizeof(int)));
         h->dtop_cap = capacity;
     }
-    CUDA_TRY(h, cudaMemsetAsync(h->dseli, 0, sizeof(int), h->stream));
-    CUDA_TRY(h, gpr::launch_collect(h->dkeys, h->N, kmin, h->dtop, capacity, h->dseli, h->stream));
-    h->launches++;
-    int cnt = 0;
-    CUDA_TRY(h, cudaMemcpyAsync(&cnt, h->dseli, sizeof cnt, cudaMemcpyDeviceToHost, h->stream));
+    CUDA_TRY(h, gpr::launch_select(h->kp, h->N - k, h->dkeys, h->dsel, h->dseli, h->hsel, h->stream));
+    CUDA_TRY(h, gpr::launch_collect(h->dkeys, h->N, h->dsel, margin, h->dtop, capacity, h->dseli, h->stream));
+    h->launches += 2;
+    /* the count and, as far as the pinned room goes, the chains in one wait */
+    int* stage = (int*)(h->hsel + 1);
+    const int ahead = std::min(capacity, GPR_TOP_STAGE);
+    CUDA_TRY(h, cudaMemcpyAsync(&h->hsel->count, h->dseli, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    if (ahead > 0)
+        CUDA_TRY(h, cudaMemcpyAsync(stage, h->dtop, (size_t)ahead * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-    const int m = cnt < capacity ? cnt : capacity;
-    if (m > 0) {
+    const int cnt = h->hsel->count;
+    if (threshold) *threshold = gpr_key_value(h->hsel->key);
+    const int m = std::min(cnt, capacity);
+    if (m > ahead) {
         CUDA_TRY(h, cudaMemcpyAsync(chains, h->dtop, (size_t)m * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
         CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-        std::sort(chains, chains + m);
+    } else if (m > 0) {
+        memcpy(chains, stage, (size_t)m * sizeof(int));
     }
+    if (m > 0) std::sort(chains, chains + m);
     *n = cnt;
     return GPR_OK;
 }
@@ -1458,17 +1459,13 @@ int gpr_map_chain(gpr_handle* h, int* chain, double* posterior) {
     if (!h) return GPR_ERR_ARG;
     if (!chain) return fail(h, GPR_ERR_ARG, "chain is NULL");
     CUDA_TRY(h, cudaSetDevice(h->device));
-    int rc = select_rank(h, h->N - 1, nullptr);
+    int rc = ensure_select(h);
     if (rc != GPR_OK) return rc;
-    const int big = 0x7fffffff;
-    CUDA_TRY(h, cudaMemcpyAsync(h->dseli + 1, &big, sizeof big, cudaMemcpyHostToDevice, h->stream));
-    CUDA_TRY(h, gpr::launch_first_index(h->dkeys, h->N, h->dsel, h->dseli + 1, h->stream));
+    CUDA_TRY(h, gpr::launch_select(h->kp, h->N - 1, h->dkeys, h->dsel, h->dseli, h->hsel, h->stream));
     h->launches++;
-    unsigned long long key = 0;
-    int idx = big;
-    CUDA_TRY(h, cudaMemcpyAsync(&key, h->dsel, sizeof key, cudaMemcpyDeviceToHost, h->stream));
-    CUDA_TRY(h, cudaMemcpyAsync(&idx, h->dseli + 1, sizeof idx, cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
+    const unsigned long long key = h->hsel->key;
+    const int idx = h->hsel->first;
     *chain = key == 0ull ? -1 : idx;
     if (posterior) *posterior = gpr_key_value(key);
     return GPR_OK;
