@@ -516,6 +516,7 @@ static int choose_launch(gpr_handle* h) {
 }
 
 /* Device layout of a dataset: x1 | y | w | sd | x2 | x3, nd_pad floats each
+ * (whole chunks of 128 points, lane by lane within a chunk: GPR_POINT_SLOT)
  * (x2, x3 only for three input variables). */
 static int set_data_body(gpr_handle* h, const float* x, const float* x2, const float* x3, const float* y,
                          const float* sd, int n);
@@ -541,21 +542,24 @@ static int set_data_body(gpr_handle* h, const float* x, const float* x2, const f
     for (int i = 0; i < n; ++i)
         if (!(sd[i] > 0.0f)) return fail(h, GPR_ERR_ARG, "sd[%d] = %g is not > 0", i, (double)sd[i]);
     CUDA_TRY(h, cudaSetDevice(h->device));
-    const int nd_pad = (n + 3) & ~3;
+    if (n > std::numeric_limits<int>::max() - GPR_CHUNK_POINTS)
+        return fail(h, GPR_ERR_ARG, "%d points are too many", n);
+    const int nd_pad = GPR_PAD_POINTS(n);
     std::vector<float> host((size_t)(three ? 6 : 4) * nd_pad, 0.0f);
     if (three)
         for (int i = 0; i < n; ++i) {
-            host[4 * (size_t)nd_pad + i] = x2[i];
-            host[5 * (size_t)nd_pad + i] = x3[i];
+            host[4 * (size_t)nd_pad + GPR_POINT_SLOT(i)] = x2[i];
+            host[5 * (size_t)nd_pad + GPR_POINT_SLOT(i)] = x3[i];
         }
     double normsum = 0.0;
     const double PIf = 3.141592653589;
     const int we = weight_exponent(sd, (size_t)n);
     for (int i = 0; i < n; ++i) {
-        host[i] = x[i];
-        host[nd_pad + i] = y[i];
-        host[2 * (size_t)nd_pad + i] = point_weight(sd[i], we);
-        host[3 * (size_t)nd_pad + i] = sd[i];
+        const size_t at = (size_t)GPR_POINT_SLOT(i);
+        host[at] = x[i];
+        host[nd_pad + at] = y[i];
+        host[2 * (size_t)nd_pad + at] = point_weight(sd[i], we);
+        host[3 * (size_t)nd_pad + at] = sd[i];
         /* the constant part of lnormalpdf (main.cu:300), per point */
         normsum += 0.5 * ((double)logf((float)(2.0 * PIf)) + 2.0 * (double)logf(sd[i]));
     }
@@ -615,11 +619,12 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
                                        h->N, n_datasets);
     const int cpd = h->N / n_datasets;
     const bool three = h->kp.nv == 3;
-    long long total = 0, maxn = 0, npad = 0;
+    long long total = 0, maxn = 0, npad = 0, nchunk = 0;
     for (int d = 0; d < n_datasets; ++d) {
         if (sizes[d] < 0) return fail(h, GPR_ERR_ARG, "sizes[%d] = %d is negative", d, sizes[d]);
         total += sizes[d];
         npad += (sizes[d] + 3) & ~3;
+        nchunk += ((long long)sizes[d] + GPR_CHUNK_POINTS - 1) / GPR_CHUNK_POINTS;
         if (sizes[d] > maxn) maxn = sizes[d];
     }
     if (npad > (1ll << 30)) return fail(h, GPR_ERR_ARG, "batched data too large");
@@ -629,7 +634,7 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
         if (!(sd[i] > 0.0f)) return fail(h, GPR_ERR_ARG, "sd[%lld] = %g is not > 0", i, (double)sd[i]);
     CUDA_TRY(h, cudaSetDevice(h->device));
     drop_graph(h);
-    const size_t T = (size_t)npad;
+    const size_t T = (size_t)nchunk * GPR_CHUNK_POINTS;   /* npad <= 2^30: at most 2^28 chunks */
     std::vector<float> host((three ? 6 : 4) * T + 4, 0.0f);
     std::vector<int> meta(3 * (size_t)n_datasets);
     std::vector<float> ns(2 * (size_t)n_datasets);
@@ -638,22 +643,23 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
     const int we = weight_exponent(sd, (size_t)total);
     size_t off = 0, src = 0;
     for (int d = 0; d < n_datasets; ++d) {
-        meta[d] = (int)off;
+        meta[d] = (int)(off / GPR_CHUNK_POINTS);
         meta[n_datasets + d] = sizes[d];
         double normsum = 0.0;
         for (int i = 0; i < sizes[d]; ++i, ++src) {
-            host[off + i] = x1[src];
-            host[T + off + i] = y[src];
-            host[2 * T + off + i] = point_weight(sd[src], we);
-            host[3 * T + off + i] = sd[src];
-            if (three) { host[4 * T + off + i] = x2[src]; host[5 * T + off + i] = x3[src]; }
+            const size_t at = off + (size_t)GPR_POINT_SLOT(i);
+            host[at] = x1[src];
+            host[T + at] = y[src];
+            host[2 * T + at] = point_weight(sd[src], we);
+            host[3 * T + at] = sd[src];
+            if (three) { host[4 * T + at] = x2[src]; host[5 * T + at] = x3[src]; }
             normsum += 0.5 * ((double)logf((float)(2.0 * PIf)) + 2.0 * (double)logf(sd[src]));   /* main.cu:300 */
         }
         ns64[d] = normsum;
         const double nsd = normsum * 0x1p-64;
         ns[2 * d] = (float)nsd;
         ns[2 * d + 1] = (float)(nsd - (double)ns[2 * d]);
-        off += (sizes[d] + 3) & ~3;
+        off += (size_t)GPR_PAD_POINTS(sizes[d]);
     }
     /* datasets claimed largest first, so that uneven sizes balance across the grid */
     std::vector<int> order(n_datasets);
@@ -677,7 +683,7 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
     CUDA_TRY(h, cudaStreamSynchronize(h->stream));
     gpr::KParams& kp = h->kp;
     h->nd = (int)maxn;
-    h->nd_pad = (int)((maxn + 3) & ~3);
+    h->nd_pad = (int)GPR_PAD_POINTS(maxn);
     kp.nd = h->nd; kp.nd_pad = h->nd_pad;
     kp.normsum_hi = kp.normsum_lo = 0.0f;
     kp.normsum64 = 0.0;
@@ -1499,17 +1505,20 @@ static std::mutex g_noalloc_mu;
 static int g_noalloc_sms[kNoallocMaxDevices];
 
 /* The weights of gpr_set_data, computed in place from sd on the device (the
- * same IEEE double operations and rounding as the host code), and zero
- * padding up to nd_pad, which the kernel stages with the data. */
-static __global__ void noalloc_data_kernel(float* x, float* y, float* w, int n, int nd_pad, double wscale) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nd_pad) return;
+ * same IEEE double operations and rounding as the host code), the points put
+ * in chunk order and zero padding up to whole chunks, which the kernel stages
+ * with the data.  One CTA of GPR_CHUNK_POINTS threads per chunk. */
+static __global__ void noalloc_data_kernel(float* x, float* y, float* w, int n, double wscale) {
+    const int i = blockIdx.x * GPR_CHUNK_POINTS + threadIdx.x;
+    float xi = 0.0f, yi = 0.0f, wi = 0.0f;
     if (i < n) {
         const double s = (double)w[i];
-        w[i] = (float)(wscale / (2.0 * s * s));
-    } else {
-        x[i] = 0.0f; y[i] = 0.0f; w[i] = 0.0f;
+        xi = x[i]; yi = y[i];
+        wi = (float)(wscale / (2.0 * s * s));
     }
+    __syncthreads();   /* in place: every point of the chunk has been read */
+    const int at = GPR_POINT_SLOT(i);
+    x[at] = xi; y[at] = yi; w[at] = wi;
 }
 
 /* Per call, with the device current: the scratch array's device address,
@@ -1655,7 +1664,7 @@ extern "C" int gpr_run_block_noalloc(const gpr_config* cfg, int n_chains, int32_
     kp.err = h.dcounter + 1;
     kp.stats = nullptr;
 
-    const int nd_pad = (ndata + 3) & ~3;
+    const int nd_pad = GPR_PAD_POINTS(ndata);
     double normsum = 0.0;
     const double PIf = 3.141592653589;
     for (int i = 0; i < ndata; ++i)
@@ -1685,7 +1694,8 @@ extern "C" int gpr_run_block_noalloc(const gpr_config* cfg, int n_chains, int32_
         NA_TRY(cudaMemcpyAsync(sx, x, ndata * sizeof(float), cudaMemcpyHostToDevice, h.stream));
         NA_TRY(cudaMemcpyAsync(sy, y, ndata * sizeof(float), cudaMemcpyHostToDevice, h.stream));
         NA_TRY(cudaMemcpyAsync(sw, sd, ndata * sizeof(float), cudaMemcpyHostToDevice, h.stream));
-        noalloc_data_kernel<<<(nd_pad + 255) / 256, 256, 0, h.stream>>>(sx, sy, sw, ndata, nd_pad, ldexp(1.0, -we));
+        noalloc_data_kernel<<<nd_pad / GPR_CHUNK_POINTS, GPR_CHUNK_POINTS, 0, h.stream>>>(sx, sy, sw, ndata,
+                                                                                          ldexp(1.0, -we));
         NA_TRY(cudaGetLastError());
     }
 #undef NA_TRY

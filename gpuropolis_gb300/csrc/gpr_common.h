@@ -148,6 +148,16 @@ enum gpr_phase {
  * into; beyond it each warp evaluates its own chain. */
 #define GPR_MAX_PASSES 64
 
+/* ---- dataset arrays ----
+ * Points are kept in chunks of 128, the unit of the likelihood's reduction
+ * tree, in which lane l holds points l, l + 32, l + 64 and l + 96.  An array
+ * is padded with zeros to whole chunks, and within a chunk lane by lane, so
+ * that a lane's four points are one 16-byte load. */
+#define GPR_CHUNK_POINTS 128
+#define GPR_PAD_POINTS(n) (((n) + GPR_CHUNK_POINTS - 1) / GPR_CHUNK_POINTS * GPR_CHUNK_POINTS)
+/* Where point i of a dataset is in its arrays. */
+#define GPR_POINT_SLOT(i) (((i) & ~127) | (((i) & 31) << 2) | (((i) >> 5) & 3))
+
 /* Maximum compiled length for a program of PL heap nodes. */
 #define GPR_MAX_INSTR(PL) (2 * (PL) + 4)
 

@@ -1,8 +1,8 @@
 /*
  * gpr_hmc.cu -- instantiations and launchers of the adjoint kernel
  * (gpr_loglik_grad) and of the MH kernel with Hamiltonian constant moves
- * (gpr_hmc.cuh).  Four points per lane; the thread-local tape holds up to
- * 130 instructions (PROGRAM_LENGTH <= 63) or 258 (PROGRAM_LENGTH <= 127); the
+ * (gpr_hmc.cuh).  The tape's thread-local part holds up to 96 rows
+ * (PROGRAM_LENGTH <= 63) or 192 (PROGRAM_LENGTH <= 127); the
  * dataset is staged per CTA or, when too large, read from device memory.
  */
 #include "gpr_hmc.cuh"
@@ -15,17 +15,17 @@ size_t grad_smem_bytes(const KParams& p, int warps_per_cta, int stream) {
            (size_t)warps_per_cta * grad_warp_bytes(p.PL, p.max_instr);
 }
 
-bool grad_supported(const KParams& p) { return p.max_instr <= 258 && p.levels <= GPR_ASTK_MAX; }
+bool grad_supported(const KParams& p) { return p.max_instr <= 258 && p.PL <= 127; }
 
-template <int MAXI, int NV>
+template <int MAXR, int NV>
 static const void* grad_kernel_nv(int stream) {
-    return stream ? (const void*)loglik_grad_kernel<GPR_HMC_K, MAXI, true, NV>
-                  : (const void*)loglik_grad_kernel<GPR_HMC_K, MAXI, false, NV>;
+    return stream ? (const void*)loglik_grad_kernel<MAXR, true, NV>
+                  : (const void*)loglik_grad_kernel<MAXR, false, NV>;
 }
 
-template <int MAXI>
+template <int MAXR>
 static const void* grad_kernel_t(int stream, int nv) {
-    return nv == 3 ? grad_kernel_v3(MAXI, stream) : grad_kernel_nv<MAXI, 1>(stream);
+    return nv == 3 ? grad_kernel_v3(MAXR, stream) : grad_kernel_nv<MAXR, 1>(stream);
 }
 
 cudaError_t launch_loglik_grad(const KParams& p, double* grad, double* lik, int stream, cudaStream_t st) {
@@ -33,7 +33,7 @@ cudaError_t launch_loglik_grad(const KParams& p, double* grad, double* lik, int 
     if (p.nds > 0) stream = 1;   /* batched data are read per chain from device memory */
     const int wpc = 4;
     const size_t smem = grad_smem_bytes(p, wpc, stream);
-    const void* f = p.max_instr <= 130 ? grad_kernel_t<130>(stream, p.nv) : grad_kernel_t<258>(stream, p.nv);
+    const void* f = p.max_instr <= 130 ? grad_kernel_t<96>(stream, p.nv) : grad_kernel_t<192>(stream, p.nv);
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     KParams pp = p;
@@ -41,16 +41,16 @@ cudaError_t launch_loglik_grad(const KParams& p, double* grad, double* lik, int 
     return cudaLaunchKernel(f, dim3((p.N + wpc - 1) / wpc), dim3(wpc * 32), args, smem, st);
 }
 
-template <int MAXI, int RNG, int NV>
+template <int MAXR, int RNG, int NV>
 static const void* hmc_kernel_t(int stream) {
-    return stream ? (const void*)mh_hmc_kernel<GPR_HMC_K, MAXI, RNG, true, NV>
-                  : (const void*)mh_hmc_kernel<GPR_HMC_K, MAXI, RNG, false, NV>;
+    return stream ? (const void*)mh_hmc_kernel<MAXR, RNG, true, NV>
+                  : (const void*)mh_hmc_kernel<MAXR, RNG, false, NV>;
 }
 
 static const void* hmc_kernel(const KParams& p, int stream) {
     if (p.nv == 3) return hmc_kernel_v3(p, stream);
-    if (p.max_instr <= 130) return p.rng_mode ? hmc_kernel_t<130, 1, 1>(stream) : hmc_kernel_t<130, 0, 1>(stream);
-    return p.rng_mode ? hmc_kernel_t<258, 1, 1>(stream) : hmc_kernel_t<258, 0, 1>(stream);
+    if (p.max_instr <= 130) return p.rng_mode ? hmc_kernel_t<96, 1, 1>(stream) : hmc_kernel_t<96, 0, 1>(stream);
+    return p.rng_mode ? hmc_kernel_t<192, 1, 1>(stream) : hmc_kernel_t<192, 0, 1>(stream);
 }
 
 /* The shared-memory share of the L1/shared array: the rest is L1, where the

@@ -4,19 +4,20 @@
  * step) instead of the reference's independence / random-walk proposals.
  *
  * Adjoint.  The compiled postfix program (gpr_common.h) is run forward once
- * per batch of K data points per lane with every instruction's result kept on
- * a tape in the thread's local memory (one 16-byte row per instruction for
- * K = 4; L1-resident for programs of realistic length, and leaving shared
- * memory to occupancy); the backward sweep then walks the instructions in reverse,
- * carrying d loglik / d acc, splitting it at each binary instruction into the
- * accumulator's and the operand's share, and adding the operand's share to
+ * per batch of K data points per lane, and the results that the way back needs
+ * are kept on a tape: rows of K values per lane in the warp's shared memory
+ * (thread-local memory for the rare program that needs more rows than a warp
+ * has).  The backward sweep walks the instructions in reverse, carrying
+ * d loglik / d acc, splitting it at each binary instruction into the
+ * accumulator's and the operand's share, and handing the operand's share to
  * the constant it read (an instruction with a constant operand, or a constant
- * load, reads exactly one heap node's constant).  A popped operand's share is
- * parked on an adjoint stack and handed back at its PUSH.  The value a POP
- * reads is the tape entry of its matching PUSH, so the forward sweep needs no
- * value stack.  d loglik / d f at a point is 2 w (y - f) with w = 1/(2 sd^2)
- * (lnormalpdf, main.cu:299-301); sums run per lane in FP32 at the
- * bookkeeping scale 2^-64 and are reduced across lanes per constant.
+ * load, reads exactly one heap node's constant).  A popped operand's share
+ * takes the place of the pushed value on the tape, until its PUSH.  The value
+ * a POP reads is the tape row of its matching PUSH, so the forward sweep needs
+ * no value stack.  d loglik / d f at a point is 2 w (y - f) with
+ * w = 1/(2 sd^2) (lnormalpdf, main.cu:299-301); sums run per lane in FP32 at
+ * the bookkeeping scale 2^-64 and are reduced across lanes per constant, 128
+ * points at a time.
  *
  * HMC move (no reference counterpart).  Momentum m ~ N(0, I) over all PL
  * constants; leapfrog with step eps, L steps, on the log-posterior
@@ -33,27 +34,55 @@
 
 namespace gpr {
 
-#define GPR_HMC_K 4          /* points per lane of the adjoint and Hamiltonian kernels */
-#define GPR_ASTK_MAX 8       /* adjoint-stack rows: value-stack depth for PROGRAM_LENGTH <= 255 */
+/* Passes of 128 points (four per lane) that one sweep takes together: the
+ * instructions are decoded once for G of them.  On the rational model (1,024
+ * points) and on 16,384 points of three variables, with registers for 16 warps
+ * per SM: 86 and 90 ms with 2, 94 and 100 ms with 1, 141 and 95 ms with 4; with
+ * registers for 24 warps 115 and 105 ms with 2, 89 and 107 ms with 1. */
+#ifndef GPR_GRAD_G
+#define GPR_GRAD_G 2
+#endif
+/* Tape rows in shared memory (of G * 512 bytes per warp). */
+#ifndef GPR_GRAD_ROWS
+#define GPR_GRAD_ROWS 4
+#endif
+/* Resident CTAs of 8 warps per SM that the registers are allocated for. */
+#ifndef GPR_HMC_MIN_CTAS
+#define GPR_HMC_MIN_CTAS 2
+#endif
+#define GPR_GRAD_CONSTS 8    /* constants whose shares are reduced together */
+#define GPR_GRAD_STRIDE 36   /* floats between their rows of lane shares: conflict-free reads of the reduction */
 
-/* One tape row: an instruction's result at this lane's K points. */
-template <int K>
-struct alignas(K == 4 ? 16 : (K == 2 ? 8 : 4)) Row {
-    float v[K];
-};
+/* The adjoint's instruction word: code and heap node as in gpr_word; the tape
+ * row that keeps the instruction's result (or, for the input variables, that
+ * it needs none); and for a binary instruction the row of the value it pops,
+ * for one that reads a constant that constant's place among those the program
+ * reads.  1 and the invalid-op marker are constants of the nodes below, which
+ * no program has (PROGRAM_LENGTH <= 127). */
+#define GW_ROW(w) (((w) >> 16) & 255u)
+#define GW_AUX(w) ((w) >> 24)
+#define GW_NONE 255u
+#define GW_X1 254u           /* the result is x1, x2, x3 */
+#define GW_X2 253u
+#define GW_X3 252u
+#define GW_NODE_ONE 254u
+#define GW_NODE_NAN 255u
 
 /* Per-warp shared memory of the gradient evaluator and the HMC kernel. */
 struct GradSmem {
     uint8_t* ops[2];
     float* Cs[2];       /* [0], [1]: current and proposed constants            */
     gpr_word* prog[2];
-    uint2* eprog;
-    int16_t* match;     /* POP instruction -> index of its PUSH                 */
-    float* gacc;        /* [PL]: the gradient sums (lane 0 adds each warp-summed
-                         * share); also the compiler's scratch                   */
+    uint32_t* gprog;    /* adjoint instruction words of the program at hand     */
+    uint2* eprog;       /* ... paired with the constants they read              */
+    uint8_t* cnode;     /* [GPR_GRAD_CONSTS]: nodes of the first constants it reads */
+    float* gacc;        /* [PL]: gradient sums of the constants beyond those (lane 0
+                         * adds each warp-summed share); also the compiler's scratch */
     float* gcur;        /* gradient of the log-posterior at the current state   */
     float* gnew;        /* ... at the trajectory's position                     */
     float* mom;         /* momentum                                             */
+    float* rows;        /* the tape: [GPR_GRAD_ROWS][G][32 lanes] of four values */
+    float* share;       /* [G * GPR_GRAD_CONSTS][GPR_GRAD_STRIDE]: lane shares   */
 };
 
 __host__ __device__ __forceinline__ size_t grad_rows_bytes(int PL) {
@@ -68,10 +97,13 @@ __host__ __device__ __forceinline__ size_t grad_warp_bytes(int PL, int max_instr
     b += 2 * plp;                                              /* ops */
     b += align16(2 * plp * 4);                                 /* Cs */
     b += align16(2 * (size_t)max_instr * sizeof(gpr_word));    /* prog */
+    b += align16((size_t)max_instr * 4);                       /* gprog */
     b += align16((size_t)max_instr * 8);                       /* eprog */
-    b += align16((size_t)max_instr * 2);                       /* match */
-    b += grad_rows_bytes(PL);                                  /* gradient rows | compiler scratch */
+    b += 16;                                                   /* cnode */
+    b += grad_rows_bytes(PL);                                  /* gradient sums | compiler scratch */
     b += 3 * align16(plp * 4);                                 /* gcur, gnew, mom */
+    b += (size_t)GPR_GRAD_ROWS * GPR_GRAD_G * 512;             /* rows */
+    b += (size_t)GPR_GRAD_G * GPR_GRAD_CONSTS * GPR_GRAD_STRIDE * 4;   /* share */
     return align16(b);
 }
 
@@ -82,291 +114,529 @@ __device__ __forceinline__ GradSmem carve_grad(uint8_t* base, int PL, int max_in
     w.ops[0] = p; w.ops[1] = p + plp; p += 2 * plp;
     w.Cs[0] = (float*)p; w.Cs[1] = (float*)p + plp; p += align16(2 * plp * 4);
     w.prog[0] = (gpr_word*)p; w.prog[1] = (gpr_word*)p + max_instr; p += align16(2 * (size_t)max_instr * sizeof(gpr_word));
+    w.gprog = (uint32_t*)p; p += align16((size_t)max_instr * 4);
     w.eprog = (uint2*)p; p += align16((size_t)max_instr * 8);
-    w.match = (int16_t*)p; p += align16((size_t)max_instr * 2);
+    w.cnode = p; p += 16;
     w.gacc = (float*)p; p += grad_rows_bytes(PL);
     w.gcur = (float*)p; p += align16(plp * 4);
     w.gnew = (float*)p; p += align16(plp * 4);
-    w.mom = (float*)p;
+    w.mom = (float*)p; p += align16(plp * 4);
+    w.rows = (float*)p; p += (size_t)GPR_GRAD_ROWS * GPR_GRAD_G * 512;
+    w.share = (float*)p;
     return w;
 }
 
-/* For each POP instruction of the program, the index of the PUSH whose value
- * it pops (the stack discipline is a property of the program alone). */
-__device__ __forceinline__ void pop_match(const gpr_word* prog, int ninstr, int16_t* match, int lane) {
+/* The adjoint words of a compiled program, into ws.gprog; returns how many
+ * constants it reads.  A result is kept only if the way back reads it: the
+ * factor of a product whose other factor is a constant or popped, an argument
+ * or a result where a derivative is written in it, and every pushed value. */
+static __device__ int grad_prepare(const gpr_word* prog, int ninstr, const GradSmem& ws, int lane) {
+    int nconst = 0;
     if (lane == 0) {
-        int16_t st[32];
-        int sp = 0;
+        uint8_t st[32];      /* instructions of the pushes pending: at most floor(log2(PL / 2)) + 1 */
+        int sp = 0, rows = 0;
+        uint32_t before = 0u;    /* the word of instruction i - 1, not stored yet */
 #pragma unroll 1
         for (int i = 0; i < ninstr; ++i) {
-            const uint32_t code = prog[i] & 0xffu;
-            if (code == I_PUSH) {
-                if (sp < 32) st[sp] = (int16_t)i;
-                ++sp;
-            } else if (code >= I_BIN0 && GPR_BIN_SRC(code) == SRC_POP) {
-                --sp;
-                match[i] = (sp >= 0 && sp < 32) ? st[sp] : (int16_t)0;
+            uint32_t code = prog[i] & 0xffu, node = (prog[i] >> 8) & 0xffu;
+            uint32_t aux = GW_NONE, row = GW_NONE;
+            bool need_arg = false, need_res = false;   /* the accumulator before, after */
+            if (code == I_LD1 || code == I_LDNAN) {
+                node = code == I_LD1 ? GW_NODE_ONE : GW_NODE_NAN;
+                code = I_LDC;
             }
+            bool takes = code == I_LDC;                 /* a constant or a popped value has a share */
+            if (code >= I_BIN0) {
+                const uint32_t bop = GPR_BIN_BOP(code), left = GPR_BIN_ACCLEFT(code);
+                uint32_t src = GPR_BIN_SRC(code);
+                if (src == SRC_ONE) { src = SRC_C; node = GW_NODE_ONE; code = GPR_BIN(bop, left, SRC_C); }
+                takes = src == SRC_POP || (src == SRC_C && node < GW_NODE_ONE);
+                if (src == SRC_POP) { --sp; aux = GW_ROW(ws.gprog[st[sp]]); }
+                if (bop == BOP_MUL) need_arg = takes;
+                else if (bop == BOP_DIV) { need_arg = !left; need_res = !left || takes; }
+                else if (bop == BOP_POW) { need_arg = left || takes; need_res = !left || takes; }
+                if (src != SRC_C) takes = false;
+            } else if (code == I_PUSH) {
+                need_res = true;
+            } else if (code >= U_INV) {
+                need_res = code == U_INV || code == U_EXP || code == U_SQRT || code == U_TAN;
+                need_arg = !need_res;
+            } else if (code == I_LDX || code == I_LDX2 || code == I_LDX3) {
+                row = code == I_LDX ? GW_X1 : code == I_LDX2 ? GW_X2 : GW_X3;
+            }
+            if (takes && node < GW_NODE_ONE) {
+                if (nconst < GPR_GRAD_CONSTS) ws.cnode[nconst] = (uint8_t)node;
+                aux = (uint32_t)nconst++;
+            }
+            if (need_arg && GW_ROW(before) == GW_NONE) before = (before & 0xff00ffffu) | ((uint32_t)rows++ << 16);
+            if (i > 0) ws.gprog[i - 1] = before;
+            if (need_res) row = (uint32_t)rows++;
+            if (code == I_PUSH) { ws.gprog[i] = row << 16; st[sp++] = (uint8_t)i; }
+            before = code | (node << 8) | (row << 16) | (aux << 24);
         }
+        ws.gprog[ninstr - 1] = before;
     }
     __syncwarp();
+    return __shfl_sync(FULLMASK, nconst, 0);
 }
 
-/* Value of an operand for instruction i: x, the constant, 1 or the popped
- * value (the tape entry of the matching PUSH). */
-template <int K, int NV>
-__device__ __forceinline__ void operand(uint32_t src, float c, int i, const int16_t* match,
-                                        const float (&x)[NV][K], const Row<K>* tape, float (&v)[K]) {
-    if (src == SRC_X) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = x[0][k];
-    } else if (NV > 1 && (src == SRC_X2 || src == SRC_X3)) {
-        const int vi = NV > 1 ? (int)(src - SRC_X2) + 1 : 0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = x[vi][k];
-    } else if (src == SRC_C) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = c;
-    } else if (src == SRC_ONE) {
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = 1.0f;
-    } else {
-        const Row<K> t = tape[match[i]];
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = t.v[k];
+/* The words paired with the constants at hand. */
+__device__ __forceinline__ void build_grad_program(const uint32_t* gprog, const float* Cs, int ninstr, uint2* eprog,
+                                                   int lane) {
+#pragma unroll 1
+    for (int i = lane; i < ninstr; i += 32) {
+        const uint32_t w = gprog[i], node = (w >> 8) & 0xffu;
+        const float c = node == GW_NODE_NAN ? __int_as_float(0x7fc00000) : node == GW_NODE_ONE ? 1.0f : Cs[node];
+        eprog[i] = make_uint2(w, __float_as_uint(c));
     }
 }
 
-/* f(x) for this lane's K points, every instruction's result kept on the tape.
- * The arithmetic is the evaluator's (run_program), operation for operation. */
+/* One copy each of the long routines, four points at a time. */
+static __device__ __noinline__ float4 pow_four(float4 u, float4 w) {
+    return make_float4(gx_pow(u.x, w.x), gx_pow(u.y, w.y), gx_pow(u.z, w.z), gx_pow(u.w, w.w));
+}
+static __device__ __noinline__ float4 log_four(float4 a) {
+    return make_float4(gx_log(a.x), gx_log(a.y), gx_log(a.z), gx_log(a.w));
+}
+/* The trigonometric ops (CUDA's math library) one point after the other: each
+ * round takes the first of the four values and puts its result last. */
+static __device__ __noinline__ float4 trig_four(uint32_t code, float4 a) {
+#pragma unroll 1
+    for (int n = 0; n < 4; ++n) {
+        float r;
+        switch (code) {
+            case U_SIN: r = sinf(a.x); break;
+            case U_ASIN: r = asinf(a.x); break;
+            case U_COS: r = cosf(a.x); break;
+            case U_ACOS: r = acosf(a.x); break;
+            case U_TAN: r = tanf(a.x); break;
+            default: r = atanf(a.x); break;
+        }
+        a = make_float4(a.y, a.z, a.w, r);
+    }
+    return a;
+}
+/* Their derivatives in the argument a (tan: in its result). */
+static __device__ __noinline__ float4 trig_slope_four(uint32_t code, float4 a) {
+#pragma unroll 1
+    for (int n = 0; n < 4; ++n) {
+        float r;
+        switch (code) {
+            case U_SIN: r = cosf(a.x); break;
+            case U_ASIN: r = __fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(a.x, a.x)))); break;
+            case U_COS: r = -sinf(a.x); break;
+            case U_ACOS: r = -__fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(a.x, a.x)))); break;
+            case U_TAN: r = __fadd_rn(1.0f, __fmul_rn(a.x, a.x)); break;
+            default: r = __fdiv_rn(1.0f, __fadd_rn(1.0f, __fmul_rn(a.x, a.x))); break;
+        }
+        a = make_float4(a.y, a.z, a.w, r);
+    }
+    return a;
+}
+
+/* The tape of one lane: GPR_GRAD_ROWS rows in shared memory, the others in
+ * thread-local memory. */
+template <int K>
+struct Tape {
+    float4* sm;          /* this lane's first four values of row 0 */
+    float4* local;
+    __device__ __forceinline__ void put(uint32_t r, const float (&v)[K]) const {
+#pragma unroll
+        for (int g = 0; g < K / 4; ++g) {
+            const float4 q = make_float4(v[4 * g], v[4 * g + 1], v[4 * g + 2], v[4 * g + 3]);
+            if (r < GPR_GRAD_ROWS) sm[(r * (K / 4) + g) * 32] = q;
+            else local[(r - GPR_GRAD_ROWS) * (K / 4) + g] = q;
+        }
+    }
+    __device__ __forceinline__ void get(uint32_t r, float (&v)[K]) const {
+#pragma unroll
+        for (int g = 0; g < K / 4; ++g) {
+            const float4 q = r < GPR_GRAD_ROWS ? sm[(r * (K / 4) + g) * 32] : local[(r - GPR_GRAD_ROWS) * (K / 4) + g];
+            v[4 * g] = q.x; v[4 * g + 1] = q.y; v[4 * g + 2] = q.z; v[4 * g + 3] = q.w;
+        }
+    }
+};
+
+/* A result kept in row r, or one of the input variables. */
 template <int K, int NV>
-__device__ __forceinline__ void forward_tape(const uint2* __restrict__ prog, int ninstr, const int16_t* match,
-                                             const float (&x)[NV][K], Row<K>* __restrict__ tape) {
-    float acc[K];
+__device__ __forceinline__ void result_of(uint32_t r, const float (&x)[NV][K], const Tape<K>& tape, float (&v)[K]) {
+    if (r < GW_X3) {
+        tape.get(r, v);
+    } else {
+        const int vi = NV > 1 ? (int)(GW_X1 - r) : 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = x[vi][k];
+    }
+}
+
+/* Value of a binary instruction's operand: an input variable, the constant or
+ * the popped value. */
+template <int K, int NV>
+__device__ __forceinline__ void operand(uint32_t w, float c, const float (&x)[NV][K], const Tape<K>& tape,
+                                        float (&v)[K]) {
+    const uint32_t src = GPR_BIN_SRC(w & 0xffu);
+    if (src == SRC_C) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = c;
+    } else if (src == SRC_POP) {
+        tape.get(GW_AUX(w), v);
+    } else {
+        const int vi = NV > 1 && src != SRC_X ? (int)(src - SRC_X2) + 1 : 0;
+#pragma unroll
+        for (int k = 0; k < K; ++k) v[k] = x[vi][k];
+    }
+}
+
+#define GPR_EACH _Pragma("unroll") for (int k = 0; k < K; ++k)
+
+template <int K>
+__device__ __forceinline__ void pow_all(const float (&u)[K], const float (&w)[K], float (&r)[K]) {
+#pragma unroll
+    for (int g = 0; g < K / 4; ++g) {
+        const float4 q = pow_four(make_float4(u[4 * g], u[4 * g + 1], u[4 * g + 2], u[4 * g + 3]),
+                                  make_float4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]));
+        r[4 * g] = q.x; r[4 * g + 1] = q.y; r[4 * g + 2] = q.z; r[4 * g + 3] = q.w;
+    }
+}
+template <int K>
+__device__ __forceinline__ void log_all(const float (&a)[K], float (&r)[K]) {
+#pragma unroll
+    for (int g = 0; g < K / 4; ++g) {
+        const float4 q = log_four(make_float4(a[4 * g], a[4 * g + 1], a[4 * g + 2], a[4 * g + 3]));
+        r[4 * g] = q.x; r[4 * g + 1] = q.y; r[4 * g + 2] = q.z; r[4 * g + 3] = q.w;
+    }
+}
+
+template <int K, bool SLOPE>
+__device__ __forceinline__ void trig_all(uint32_t code, const float (&a)[K], float (&r)[K]) {
+#pragma unroll
+    for (int g = 0; g < K / 4; ++g) {
+        const float4 u = make_float4(a[4 * g], a[4 * g + 1], a[4 * g + 2], a[4 * g + 3]);
+        const float4 q = SLOPE ? trig_slope_four(code, u) : trig_four(code, u);
+        r[4 * g] = q.x; r[4 * g + 1] = q.y; r[4 * g + 2] = q.z; r[4 * g + 3] = q.w;
+    }
+}
+
+/* acc = f(x) for this lane's K points, the results that the way back needs
+ * kept on the tape.  The arithmetic is the evaluator's (run_program),
+ * operation for operation. */
+template <int K, int NV>
+__device__ __forceinline__ void forward_tape(const uint2* __restrict__ prog, int ninstr, const float (&x)[NV][K],
+                                             const Tape<K>& tape, float (&acc)[K]) {
 #pragma unroll
     for (int k = 0; k < K; ++k) acc[k] = 0.0f;
+    uint2 nxt = prog[0];
 #pragma unroll 1
     for (int i = 0; i < ninstr - 1; ++i) {
-        const uint2 insw = prog[i];
-        const uint32_t code = insw.x & 0xffu;
-        const float c = __uint_as_float(insw.y);
+        const uint32_t w = nxt.x, code = w & 0xffu;
+        const float c = __uint_as_float(nxt.y);
+        nxt = prog[i + 1];
         if (code >= I_BIN0) {
-            const uint32_t bop = GPR_BIN_BOP(code);
-            const uint32_t accleft = GPR_BIN_ACCLEFT(code);
-            float v[K];
-            operand<K, NV>(GPR_BIN_SRC(code), c, i, match, x, tape, v);
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const float u = accleft ? acc[k] : v[k];
-                const float w = accleft ? v[k] : acc[k];
-                float r;
-                if (bop == BOP_ADD) r = __fadd_rn(acc[k], v[k]);
-                else if (bop == BOP_MUL) r = __fmul_rn(acc[k], v[k]);
-                else if (bop == BOP_SUB) r = __fsub_rn(u, w);
-                else if (bop == BOP_DIV) r = __fdiv_rn(u, w);
-                else r = gx_pow(u, w);
-                acc[k] = r;
-            }
-        } else {
-            switch (code) {
-                case I_LDX:
-#pragma unroll
-                    for (int k = 0; k < K; ++k) acc[k] = x[0][k];
-                    break;
-                case I_LDX2:
-                case I_LDX3: {
-                    const int vi = NV > 1 ? (code == I_LDX2 ? 1 : 2) : 0;
-#pragma unroll
-                    for (int k = 0; k < K; ++k) acc[k] = NV > 1 ? x[vi][k] : 0.0f;
-                    break;
+            const uint32_t bop = GPR_BIN_BOP(code), src = GPR_BIN_SRC(code);
+            const bool left = GPR_BIN_ACCLEFT(code);
+            if (bop <= BOP_MUL && src == SRC_C) {
+                if (bop == BOP_ADD) { GPR_EACH acc[k] = __fadd_rn(acc[k], c); }
+                else if (bop == BOP_MUL) { GPR_EACH acc[k] = __fmul_rn(acc[k], c); }
+                else if (left) { GPR_EACH acc[k] = __fsub_rn(acc[k], c); }
+                else { GPR_EACH acc[k] = __fsub_rn(c, acc[k]); }
+            } else if (bop <= BOP_MUL && src == SRC_X) {
+                if (bop == BOP_ADD) { GPR_EACH acc[k] = __fadd_rn(acc[k], x[0][k]); }
+                else if (bop == BOP_MUL) { GPR_EACH acc[k] = __fmul_rn(acc[k], x[0][k]); }
+                else if (left) { GPR_EACH acc[k] = __fsub_rn(acc[k], x[0][k]); }
+                else { GPR_EACH acc[k] = __fsub_rn(x[0][k], acc[k]); }
+            } else {
+                float v[K];
+                operand<K, NV>(w, c, x, tape, v);
+                if (bop == BOP_ADD) { GPR_EACH acc[k] = __fadd_rn(acc[k], v[k]); }
+                else if (bop == BOP_MUL) { GPR_EACH acc[k] = __fmul_rn(acc[k], v[k]); }
+                else {
+                    if (!left) { GPR_EACH { const float t = acc[k]; acc[k] = v[k]; v[k] = t; } }
+                    if (bop == BOP_SUB) { GPR_EACH acc[k] = __fsub_rn(acc[k], v[k]); }
+                    else if (bop == BOP_DIV) { GPR_EACH acc[k] = __fdiv_rn(acc[k], v[k]); }
+                    else pow_all<K>(acc, v, acc);
                 }
-                case I_LDC:
-#pragma unroll
-                    for (int k = 0; k < K; ++k) acc[k] = c;
-                    break;
-                case I_LD1:
-#pragma unroll
-                    for (int k = 0; k < K; ++k) acc[k] = 1.0f;
-                    break;
-                case I_LDNAN:
-#pragma unroll
-                    for (int k = 0; k < K; ++k) acc[k] = __int_as_float(0x7fc00000);
-                    break;
-                case I_PUSH: break;
-                default:
-#pragma unroll 1
-                    for (int k = 0; k < K; ++k) {
-                        const float a = acc[k];
-                        float r;
-                        switch (code) {
-                            case U_INV: r = __fdiv_rn(1.0f, a); break;
-                            case U_LOG: r = gx_log(a); break;
-                            case U_EXP: r = gx_exp(a); break;
-                            case U_SQRT: r = __fsqrt_rn(a); break;
-                            case U_SIN: r = sinf(a); break;
-                            case U_ASIN: r = asinf(a); break;
-                            case U_COS: r = cosf(a); break;
-                            case U_ACOS: r = acosf(a); break;
-                            case U_TAN: r = tanf(a); break;
-                            case U_ATAN: r = atanf(a); break;
-                            default: r = fabsf(a); break;
-                        }
-                        acc[k] = r;
-                    }
-                    break;
             }
-        }
-        Row<K> row;
+        } else if (code >= U_INV) {
+            if (code == U_EXP) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) row.v[k] = acc[k];
-        tape[i] = row;
+                for (int k = 0; k < K; ++k) acc[k] = gx_exp(acc[k]);
+            } else if (code == U_LOG) {
+                log_all<K>(acc, acc);
+            } else if (code == U_INV) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) acc[k] = __fdiv_rn(1.0f, acc[k]);
+            } else if (code == U_SQRT) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) acc[k] = __fsqrt_rn(acc[k]);
+            } else if (code == U_ABS) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) acc[k] = fabsf(acc[k]);
+            } else {
+                trig_all<K, false>(code, acc, acc);
+            }
+        } else if (code == I_LDC) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) acc[k] = c;
+        } else if (code != I_PUSH) {
+            const int vi = NV > 1 && code != I_LDX ? (code == I_LDX2 ? 1 : 2) : 0;
+#pragma unroll
+            for (int k = 0; k < K; ++k) acc[k] = x[vi][k];
+        }
+        const uint32_t row = GW_ROW(w);
+        if (row < GW_X3) tape.put(row, acc);
     }
 }
 
 /* adj * d, where a zero adjoint contributes zero even through a partial that
  * left the FP32 range (0 * inf would poison the sums). */
-__device__ __forceinline__ float adj_mul(float adj, float d) { return adj == 0.0f ? 0.0f : __fmul_rn(adj, d); }
+__device__ __forceinline__ float adj_mul(float adj, float d) {
+    float r = adj;
+    if (adj != 0.0f) r = __fmul_rn(adj, d);
+    return r;
+}
 
-/* The backward sweep: adj holds d loglik / d f per point on entry; the
- * per-constant shares are added to this lane's gradient rows. */
-template <int K, int NV>
-__device__ __forceinline__ void backward_tape(const uint2* __restrict__ prog, int ninstr, const int16_t* match,
-                                              const float (&x)[NV][K], const Row<K>* __restrict__ tape,
-                                              float (&adj)[K], Row<K>* __restrict__ astk, float* __restrict__ gacc,
-                                              int PL, int lane) {
-    int sp = 0;
-#pragma unroll 1
-    for (int i = ninstr - 2; i >= 0; --i) {
-        const uint2 insw = prog[i];
-        const uint32_t code = insw.x & 0xffu;
-        const uint32_t node = (insw.x >> 8) & 0xffu;
-        const float c = __uint_as_float(insw.y);
-        if (code >= I_BIN0) {
-            const uint32_t bop = GPR_BIN_BOP(code);
-            const uint32_t accleft = GPR_BIN_ACCLEFT(code);
-            const uint32_t src = GPR_BIN_SRC(code);
-            float v[K];
-            operand<K, NV>(src, c, i, match, x, tape, v);
-            float share = 0.0f;
-            /* the accumulator's input; the result only where a partial needs it */
-            const Row<K> ain = tape[i - 1];
-            Row<K> rres;
-            if (bop == BOP_DIV || bop == BOP_POW) rres = tape[i];
-            Row<K> spill;
+/* This lane's share of constant number j: the sum over each pass's four
+ * points.  The first GPR_GRAD_CONSTS constants leave it for reduce_shares; the
+ * others are summed over the warp at once. */
+template <int K>
+__device__ __forceinline__ void give_share(const float (&av)[K], uint32_t w, const GradSmem& ws, int lane) {
+    const uint32_t j = GW_AUX(w);
+    if (j == GW_NONE) return;
+    float s[K / 4];
 #pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const float a = ain.v[k];
-                const float res = (bop == BOP_DIV || bop == BOP_POW) ? rres.v[k] : 0.0f;
-                const float u = accleft ? a : v[k];
-                const float w = accleft ? v[k] : a;
-                float du, dw;
-                if (bop == BOP_ADD) { du = 1.0f; dw = 1.0f; }
-                else if (bop == BOP_SUB) { du = 1.0f; dw = -1.0f; }
-                else if (bop == BOP_MUL) { du = w; dw = u; }
-                else if (bop == BOP_DIV) { du = __fdiv_rn(1.0f, w); dw = -__fdiv_rn(res, w); }
-                else {
-                    du = __fmul_rn(w, gx_pow(u, __fsub_rn(w, 1.0f)));
-                    dw = res == 0.0f ? 0.0f : __fmul_rn(res, gx_log(u));
-                }
-                const float au = adj_mul(adj[k], du), aw = adj_mul(adj[k], dw);
-                const float av = accleft ? aw : au;
-                adj[k] = accleft ? au : aw;
-                spill.v[k] = av;
-                share = __fadd_rn(share, av);
-            }
-            if (src == SRC_POP) astk[sp++] = spill;
-            else if (src == SRC_C && (int)node < PL) {
-                const float tot = warp_sum(share);
-                if (lane == 0) gacc[node] += tot;
-            }
-        } else if (code == I_LDC) {
-            float share = 0.0f;
+    for (int g = 0; g < K / 4; ++g)
+        s[g] = __fadd_rn(__fadd_rn(__fadd_rn(av[4 * g], av[4 * g + 1]), av[4 * g + 2]), av[4 * g + 3]);
+    if (j < GPR_GRAD_CONSTS) {
+        float* q = ws.share + (int)j * GPR_GRAD_STRIDE + lane;
 #pragma unroll
-            for (int k = 0; k < K; ++k) { share = __fadd_rn(share, adj[k]); adj[k] = 0.0f; }
-            if ((int)node < PL) {
-                const float tot = warp_sum(share);
-                if (lane == 0) gacc[node] += tot;
-            }
-        } else if (code == I_LDX || code == I_LD1 || code == I_LDNAN || code == I_LDX2 || code == I_LDX3) {
+        for (int g = 0; g < K / 4; ++g) q[g * GPR_GRAD_CONSTS * GPR_GRAD_STRIDE] = s[g];
+    } else {
 #pragma unroll
-            for (int k = 0; k < K; ++k) adj[k] = 0.0f;
-        } else if (code == I_PUSH) {
-            const Row<K> t = astk[--sp];
-#pragma unroll
-            for (int k = 0; k < K; ++k) adj[k] = t.v[k];
-        } else {
-            const Row<K> ain = tape[i - 1], rres = tape[i];
-#pragma unroll 1
-            for (int k = 0; k < K; ++k) {
-                const float a = ain.v[k];
-                const float res = rres.v[k];
-                float d;
-                switch (code) {
-                    case U_INV: d = -__fmul_rn(res, res); break;
-                    case U_LOG: d = __fdiv_rn(1.0f, a); break;
-                    case U_EXP: d = res; break;
-                    case U_SQRT: d = __fdiv_rn(0.5f, res); break;
-                    case U_SIN: d = cosf(a); break;
-                    case U_ASIN: d = __fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(a, a)))); break;
-                    case U_COS: d = -sinf(a); break;
-                    case U_ACOS: d = -__fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(a, a)))); break;
-                    case U_TAN: d = __fadd_rn(1.0f, __fmul_rn(res, res)); break;
-                    case U_ATAN: d = __fdiv_rn(1.0f, __fadd_rn(1.0f, __fmul_rn(a, a))); break;
-                    default: d = a > 0.0f ? 1.0f : (a < 0.0f ? -1.0f : 0.0f); break;
-                }
-                adj[k] = adj_mul(adj[k], d);
-            }
+        for (int g = 0; g < K / 4; ++g) {
+            const float tot = warp_sum(s[g]);
+            if (lane == 0) ws.gacc[(w >> 8) & 0xffu] += tot;
         }
     }
+}
+
+/* The backward sweep: adj holds d loglik / d f per point on entry. */
+template <int K, int NV>
+__device__ __forceinline__ void backward_tape(const uint2* __restrict__ prog, int ninstr, const float (&x)[NV][K],
+                                              const Tape<K>& tape, float (&adj)[K], const GradSmem& ws, int lane) {
+    uint2 nxt = prog[ninstr - 2];
+#pragma unroll 1
+    for (int i = ninstr - 2; i >= 0; --i) {
+        const uint32_t w = nxt.x, code = w & 0xffu;
+        const float c = __uint_as_float(nxt.y);
+        nxt = prog[i > 0 ? i - 1 : 0];
+        const uint32_t arg = GW_ROW(nxt.x);       /* where the accumulator before this instruction is */
+        if (code >= I_BIN0) {
+            const uint32_t bop = GPR_BIN_BOP(code), src = GPR_BIN_SRC(code);
+            const bool left = GPR_BIN_ACCLEFT(code);
+            if (bop == BOP_ADD) {
+                if (src == SRC_C) give_share<K>(adj, w, ws, lane);
+                else if (src == SRC_POP) tape.put(GW_AUX(w), adj);   /* the pushed value is done with */
+                continue;
+            }
+            if (bop == BOP_MUL && src == SRC_X) {
+                GPR_EACH adj[k] = adj_mul(adj[k], x[0][k]);
+                continue;
+            }
+            if (bop == BOP_MUL && src == SRC_C) {
+                if (arg != GW_NONE && GW_AUX(w) != GW_NONE) {
+                    float a[K];
+                    result_of<K, NV>(arg, x, tape, a);
+                    GPR_EACH a[k] = adj_mul(adj[k], a[k]);
+                    give_share<K>(a, w, ws, lane);
+                }
+                GPR_EACH adj[k] = adj_mul(adj[k], c);
+                continue;
+            }
+            const bool takes = src == SRC_C || src == SRC_POP;
+            float av[K];          /* the operand's share per point */
+            if (bop == BOP_SUB) {
+                GPR_EACH av[k] = -adj[k];
+                if (!left) { GPR_EACH { const float t = av[k]; av[k] = adj[k]; adj[k] = t; } }
+            } else {
+                float v[K];
+                operand<K, NV>(w, c, x, tape, v);
+                if (bop == BOP_MUL) {
+                    if (takes && arg != GW_NONE) {
+                        result_of<K, NV>(arg, x, tape, av);
+                        GPR_EACH av[k] = adj_mul(adj[k], av[k]);
+                    }
+                    GPR_EACH adj[k] = adj_mul(adj[k], v[k]);
+                } else {
+                    float a[K], res[K];
+                    if (arg != GW_NONE) result_of<K, NV>(arg, x, tape, a);
+                    if (GW_ROW(w) < GW_X3) tape.get(GW_ROW(w), res);
+                    if (bop == BOP_DIV) {
+                        /* u / w: du = 1 / w, dw = -res / w */
+                        if (!left) { GPR_EACH v[k] = a[k]; }
+                        float du[K], dw[K];
+                        if (left || takes) { GPR_EACH du[k] = __fdiv_rn(1.0f, v[k]); }
+                        if (!left || takes) { GPR_EACH dw[k] = -__fdiv_rn(res[k], v[k]); }
+                        if (left) {
+                            GPR_EACH { av[k] = adj_mul(adj[k], dw[k]); adj[k] = adj_mul(adj[k], du[k]); }
+                        } else {
+                            GPR_EACH { av[k] = adj_mul(adj[k], du[k]); adj[k] = adj_mul(adj[k], dw[k]); }
+                        }
+                    } else {
+                        /* u^w: du = w u^(w - 1), dw = u^w log u */
+                        if (!left) { GPR_EACH { const float t = a[k]; a[k] = v[k]; v[k] = t; } }
+                        float du[K], dw[K];
+                        if (left || takes) {
+                            float e[K];
+                            GPR_EACH e[k] = __fsub_rn(v[k], 1.0f);
+                            pow_all<K>(a, e, du);
+                            GPR_EACH du[k] = __fmul_rn(v[k], du[k]);
+                        }
+                        if (!left || takes) {
+                            log_all<K>(a, dw);
+                            GPR_EACH dw[k] = res[k] == 0.0f ? 0.0f : __fmul_rn(res[k], dw[k]);
+                        }
+                        if (left) {
+                            GPR_EACH { av[k] = adj_mul(adj[k], dw[k]); adj[k] = adj_mul(adj[k], du[k]); }
+                        } else {
+                            GPR_EACH { av[k] = adj_mul(adj[k], du[k]); adj[k] = adj_mul(adj[k], dw[k]); }
+                        }
+                    }
+                }
+            }
+            if (src == SRC_POP) tape.put(GW_AUX(w), av);
+            else if (src == SRC_C) give_share<K>(av, w, ws, lane);
+        } else if (code == I_PUSH) {
+            tape.get(GW_ROW(w), adj);
+        } else if (code >= U_INV) {
+            float a[K], res[K];
+            if (arg != GW_NONE) result_of<K, NV>(arg, x, tape, a);
+            if (GW_ROW(w) < GW_X3) tape.get(GW_ROW(w), res);
+            if (code == U_EXP) { GPR_EACH adj[k] = adj_mul(adj[k], res[k]); }
+            else if (code == U_INV) { GPR_EACH adj[k] = adj_mul(adj[k], -__fmul_rn(res[k], res[k])); }
+            else if (code == U_LOG) { GPR_EACH adj[k] = adj_mul(adj[k], __fdiv_rn(1.0f, a[k])); }
+            else if (code == U_SQRT) { GPR_EACH adj[k] = adj_mul(adj[k], __fdiv_rn(0.5f, res[k])); }
+            else if (code == U_ABS) {
+                GPR_EACH adj[k] = adj_mul(adj[k], a[k] > 0.0f ? 1.0f : (a[k] < 0.0f ? -1.0f : 0.0f));
+            } else {
+                if (code == U_TAN) { GPR_EACH a[k] = res[k]; }
+                trig_all<K, true>(code, a, a);
+                GPR_EACH adj[k] = adj_mul(adj[k], a[k]);
+            }
+        } else if (code == I_LDC) {
+            give_share<K>(adj, w, ws, lane);
+        }
+    }
+}
+
+/* The lane shares of pass group g summed over the warp, constant j in the
+ * four lanes 4j .. 4j + 3: the tree of an xor butterfly (distances 16, 8, 4,
+ * 2, 1) for all constants at once, where one butterfly after the other takes
+ * ten instructions each. */
+__device__ __forceinline__ float reduce_shares(const float* share, int g, int lane) {
+    const float* p = share + (g * GPR_GRAD_CONSTS + (lane >> 2)) * GPR_GRAD_STRIDE + (lane & 3);
+    const float t0 = __fadd_rn(p[0], p[16]), t1 = __fadd_rn(p[4], p[20]);
+    const float t2 = __fadd_rn(p[8], p[24]), t3 = __fadd_rn(p[12], p[28]);
+    float v = __fadd_rn(__fadd_rn(t0, t2), __fadd_rn(t1, t3));
+    v = __fadd_rn(v, __shfl_xor_sync(FULLMASK, v, 2));
+    return __fadd_rn(v, __shfl_xor_sync(FULLMASK, v, 1));
 }
 
 /* Log-likelihood of one program (double-float at scale 2^-64, -inf when any
  * point is invalid, as eval_loglik) and its gradient over all PL constants:
  * g[i] = 2^-64 d loglik / d C[i] in FP32, at the bookkeeping scale like the
  * likelihood (0 for constants the program does not read).  The gradient is
- * meaningful only when the likelihood is finite. */
-template <int K, int MAXI, int NV, bool STREAM>
-__device__ df eval_loglik_grad(const uint2* prog, int ninstr, const GradSmem& ws, const DataView& dv,
-                               const KParams& p, int lane, int& pts, float* g) {
+ * meaningful only when the likelihood is finite.  nconst: constants the
+ * program reads (grad_prepare).
+ *
+ * Bound by issued instructions, most of them the interpreter's, and by their
+ * latency: hence only the rows that are read again are kept, and in shared
+ * memory (a row for every instruction in thread-local memory made 8 GB of
+ * DRAM writes per 44 ms), an instruction is decoded once for G passes, sums
+ * and products with a constant or x take their operand where it is, and the
+ * constants' shares are reduced together.  65,536 chains of the rational model,
+ * 1,024 points, 10 moves of 8 leapfrog steps: 146 -> 82 ms; their gradients
+ * alone 1.86 -> 1.0 ms. */
+template <int MAXR, int NV, bool STREAM>
+static __device__ __noinline__ df eval_loglik_grad(const uint2* prog, int ninstr, int nconst, const GradSmem ws,
+                                                   const DataView dv, const KParams& p, int lane, int& pts_out,
+                                                   float* g) {
+    constexpr int G = GPR_GRAD_G, K = 4 * G;
     const int PL = p.PL;
-    Row<K> tape[MAXI];             /* thread-local: results of every instruction */
-    Row<K> astk[GPR_ASTK_MAX];     /* adjoints of pushed values                  */
+    float4 local_rows[MAXR * G];   /* rows beyond the warp's: a program of PL nodes keeps at most 3 PL / 2 */
+    Tape<K> tape;
+    tape.sm = (float4*)ws.rows + lane;
+    tape.local = local_rows;
 #pragma unroll 1
     for (int j = lane; j < PL; j += 32) ws.gacc[j] = 0.0f;
     __syncwarp();
+    const float w_to_df = p.w_to_df;
+    int pts = 0;
     float s = 0.0f;
+    float mine = 0.0f;             /* lanes 4j..4j+3: the sum of constant j */
     bool bad = false;
-    const int npass = (dv.nd + 32 * K - 1) / (32 * K);
+    const int npass = (dv.nd + 127) / 128;
 #pragma unroll 1
-    for (int pass = 0; pass < npass && !bad; ++pass) {
+    for (int pass = 0; pass < npass && !bad; pass += G) {
         float x[NV][K], adj[K];
-        const int base = pass * 32 * K + lane;
-        const uint32_t valid = load_points<K, NV, STREAM>(dv, p, base, x);
-        forward_tape<K, NV>(prog, ninstr, ws.match, x, tape);
-        pts += min(32 * K, dv.nd - pass * 32 * K);
-        const Row<K> fres = tape[ninstr - 2];
+        load_points<K, NV, STREAM>(dv, pass, lane, x);
+        forward_tape<K, NV>(prog, ninstr, x, tape, adj);
+        int good = 0;              /* passes before the first with an invalid point */
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            adj[k] = 0.0f;
-            if (valid & (1u << k)) {
-                const int i = base + 32 * k;
-                const float f = fres.v[k];
+        for (int gi = 0; gi < G; ++gi) {
+            const int left = dv.nd - (pass + gi) * GPR_CHUNK_POINTS;
+            if (bad || left <= 0) {
+#pragma unroll
+                for (int k = 4 * gi; k < 4 * gi + 4; ++k) adj[k] = 0.0f;
+                continue;
+            }
+            const float4 y4 = data_at<STREAM>(dv, DA_Y, pass + gi, lane), w4 = data_at<STREAM>(dv, DA_W, pass + gi, lane);
+            const float y[4] = {y4.x, y4.y, y4.z, y4.w}, w[4] = {w4.x, w4.y, w4.z, w4.w};
+            bool b = false;
+            auto term = [&](int kk) {
                 /* the 2^-64-scaled weight: dw carries 2^-e; the factor 2^(e-64) is exact */
-                const float wi = __fmul_rn(data_at<STREAM>(dv, DA_W, i), p.w_to_df);
-                const float r = __fsub_rn(f, data_at<STREAM>(dv, DA_Y, i));
+                const float wi = __fmul_rn(w[kk], w_to_df);
+                const float r = __fsub_rn(adj[4 * gi + kk], y[kk]);
                 const float q = __fmul_rn(r, r);
-                bad |= !(q <= FLT_MAX);
+                b |= !(q <= FLT_MAX);
                 s = fmaf(q, wi, s);
-                adj[k] = __fmul_rn(__fmul_rn(-2.0f, wi), r);
+                adj[4 * gi + kk] = __fmul_rn(__fmul_rn(-2.0f, wi), r);
+            };
+            if (left >= GPR_CHUNK_POINTS) {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) term(kk);
+            } else {
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    if (lane + 32 * kk < left) term(kk);
+                    else adj[4 * gi + kk] = 0.0f;
+                }
+            }
+            pts += min(GPR_CHUNK_POINTS, left);
+            bad = __any_sync(FULLMASK, b);
+            if (bad) {
+#pragma unroll
+                for (int k = 4 * gi; k < 4 * gi + 4; ++k) adj[k] = 0.0f;
+            } else {
+                good = gi + 1;
             }
         }
-        bad = __any_sync(FULLMASK, bad);
-        if (!bad) backward_tape<K, NV>(prog, ninstr, ws.match, x, tape, adj, astk, ws.gacc, PL, lane);
+        if (good > 0) {
+            backward_tape<K, NV>(prog, ninstr, x, tape, adj, ws, lane);
+            if (nconst > 0) {
+                __syncwarp();
+#pragma unroll
+                for (int gi = 0; gi < G; ++gi) mine = __fadd_rn(mine, reduce_shares(ws.share, gi, lane));
+                __syncwarp();
+            }
+        }
     }
     __syncwarp();
 #pragma unroll 1
     for (int c = lane; c < PL; c += 32) g[c] = ws.gacc[c];
     __syncwarp();
+    if ((lane & 3) == 0 && (lane >> 2) < nconst) g[ws.cnode[lane >> 2]] = mine;
+    __syncwarp();
+    pts_out = pts;
     if (bad) return df_make(-INFINITY, 0.0f);
     df S = warp_sum_df(df_make(s, 0.0f));
     if (!isfinite(S.hi)) return df_make(-INFINITY, 0.0f);
@@ -415,8 +685,8 @@ __device__ __forceinline__ uint8_t* grad_dataset(uint8_t* smem, const KParams& p
     return smem + GPR_STAGED_OFFSET + align16((size_t)data_arrays(p) * p.nd_pad * 4);
 }
 
-template <int K, int MAXI, bool STREAM, int NV>
-__global__ void __launch_bounds__(128) loglik_grad_kernel(const __grid_constant__ KParams p, double* grad,
+template <int MAXR, bool STREAM, int NV>
+__global__ void __launch_bounds__(128, 2 * GPR_HMC_MIN_CTAS) loglik_grad_kernel(const __grid_constant__ KParams p, double* grad,
                                                           double* lik_out) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31;
@@ -437,10 +707,11 @@ __global__ void __launch_bounds__(128) loglik_grad_kernel(const __grid_constant_
     __syncwarp();
     const CompileOut co = compile_parallel<NV>(ws.ops[0], PL, ws.prog[0], compile_scratch(ws.gacc, PL), lane);
     __syncwarp();
-    build_eval_program(ws.prog[0], ws.Cs[0], co.ninstr, ws.eprog, lane);
-    pop_match(ws.prog[0], co.ninstr, ws.match, lane);
+    const int nconst = grad_prepare(ws.prog[0], co.ninstr, ws, lane);
+    build_grad_program(ws.gprog, ws.Cs[0], co.ninstr, ws.eprog, lane);
+    __syncwarp();
     int pts = 0;
-    const df lik = eval_loglik_grad<K, MAXI, NV, STREAM>(ws.eprog, co.ninstr, ws, dv, p, lane, pts, ws.gnew);
+    const df lik = eval_loglik_grad<MAXR, NV, STREAM>(ws.eprog, co.ninstr, nconst, ws, dv, p, lane, pts, ws.gnew);
     for (int i = lane; i < PL; i += 32) grad[(size_t)i * p.N + chain] = (double)ws.gnew[i] * GPR_DF_UNSCALE;
     if (lane == 0) lik_out[chain] = df_to_double_unscaled(lik);
 }
@@ -449,8 +720,8 @@ __global__ void __launch_bounds__(128) loglik_grad_kernel(const __grid_constant_
 /* The MH block with Hamiltonian constant moves.  One warp per chain, chains
  * claimed from the global counter; evaluation with the adjoint on K points
  * per lane. */
-template <int K, int MAXI, int RNG, bool STREAM, int NV>
-__global__ void __launch_bounds__(256) mh_hmc_kernel(const __grid_constant__ KParams p) {
+template <int MAXR, int RNG, bool STREAM, int NV>
+__global__ void __launch_bounds__(256, GPR_HMC_MIN_CTAS) mh_hmc_kernel(const __grid_constant__ KParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -493,7 +764,8 @@ __global__ void __launch_bounds__(256) mh_hmc_kernel(const __grid_constant__ KPa
         const float mu = logf(__fmul_rn(10.0f, eps0));
         int n_adapt = 0;
 
-        int cur = 0, ccur = 0, cur_count = 0, cur_ninstr = 0;
+        int cur = 0, gcur = 0, ccur = 0, cur_count = 0, cur_ninstr = 0;   /* ops, program, constants buffers */
+        int nconst = 0, prepared = -1;   /* of the program whose adjoint words ws.gprog holds, and its buffer */
         float cur_len = 0.0f;
         df cur_prior = df_make(0.f, 0.f), cur_lik = df_make(0.f, 0.f), cur_post = df_make(0.f, 0.f);
         df cur_cs = df_make(0.f, 0.f);
@@ -506,23 +778,31 @@ __global__ void __launch_bounds__(256) mh_hmc_kernel(const __grid_constant__ KPa
             const bool structural = init || (p.struct_every > 0 && step % p.struct_every == 0);
             if (structural) {
                 /* the reference's structure move (or the initial evaluation) */
-                int pbuf = cur;
+                int pbuf = cur, gbuf = gcur;
                 df forward = df_make(0.f, 0.f);
+                bool changed = true;   /* the proposal's program is not the current one (mh_block_kernel) */
                 if (!init) {
                     forward = df_make(__fmul_rn(-p.logcount[cur_count], GPR_DF_SCALE), 0.0f);
-                    structure_move<RNG>(r, ws.ops[cur], ws.ops[cur ^ 1], df_invalid(cur_post), p, ljump, lane);
+                    changed = structure_move<RNG>(r, ws.ops[cur], ws.ops[cur ^ 1], df_invalid(cur_post), p, ljump, lane);
                     pbuf = cur ^ 1;
+                    if (changed) gbuf = gcur ^ 1;
                 }
                 __syncwarp();
-                const CompileOut co = compile_parallel<NV>(ws.ops[pbuf], PL, ws.prog[pbuf],
-                                                       compile_scratch(ws.gacc, PL), lane);
-                __syncwarp();
-                const df backward = df_make(__fmul_rn(-p.logcount[co.count], GPR_DF_SCALE), 0.0f);
+                CompileOut co;
+                co.ninstr = cur_ninstr; co.length = cur_len; co.count = cur_count;
                 const df cs = init ? cauchy_sum(ws.Cs[ccur], p, lane) : cur_cs;
-                build_eval_program(ws.prog[pbuf], ws.Cs[ccur], co.ninstr, ws.eprog, lane);
-                pop_match(ws.prog[pbuf], co.ninstr, ws.match, lane);
+                df lik = cur_lik;
                 int pe = 0;
-                const df lik = eval_loglik_grad<K, MAXI, NV, STREAM>(ws.eprog, co.ninstr, ws, dv, p, lane, pe, ws.gnew);
+                if (changed) {
+                    co = compile_parallel<NV>(ws.ops[pbuf], PL, ws.prog[gbuf], compile_scratch(ws.gacc, PL), lane);
+                    __syncwarp();
+                    nconst = grad_prepare(ws.prog[gbuf], co.ninstr, ws, lane);
+                    prepared = gbuf;
+                    build_grad_program(ws.gprog, ws.Cs[ccur], co.ninstr, ws.eprog, lane);
+                    __syncwarp();
+                    lik = eval_loglik_grad<MAXR, NV, STREAM>(ws.eprog, co.ninstr, nconst, ws, dv, p, lane, pe, ws.gnew);
+                }
+                const df backward = df_make(__fmul_rn(-p.logcount[co.count], GPR_DF_SCALE), 0.0f);
                 st_pts += (unsigned)pe;
                 const df prior = df_add(length_prior(co.length, p), cs);
                 const df post = df_add(prior, lik);
@@ -533,10 +813,11 @@ __global__ void __launch_bounds__(256) mh_hmc_kernel(const __grid_constant__ KPa
                     st_sp++; st_sa += accept;
                 }
                 if (accept) {
-                    cur = pbuf; cur_len = co.length; cur_count = co.count; cur_ninstr = co.ninstr; cur_cs = cs;
+                    cur = pbuf; gcur = gbuf; cur_len = co.length; cur_count = co.count; cur_ninstr = co.ninstr; cur_cs = cs;
                     cur_prior = prior; cur_lik = lik; cur_post = post;
-                    for (int i = lane; i < PL; i += 32)
-                        ws.gcur[i] = __fadd_rn(__fmul_rn(ws.gnew[i], unscale), dcauchy(ws.Cs[ccur][i]));
+                    if (changed)
+                        for (int i = lane; i < PL; i += 32)
+                            ws.gcur[i] = __fadd_rn(__fmul_rn(ws.gnew[i], unscale), dcauchy(ws.Cs[ccur][i]));
                 }
                 __syncwarp();
             } else {
@@ -558,9 +839,12 @@ __global__ void __launch_bounds__(256) mh_hmc_kernel(const __grid_constant__ KPa
                         }
                     }
                     const float heps = __fmul_rn(0.5f, eps);
-                    /* the last structure step may have left match[] for a
-                     * rejected proposal: rebuild it for the current program */
-                    pop_match(ws.prog[cur], cur_ninstr, ws.match, lane);
+                    /* the last structure step may have left the adjoint words of a
+                     * rejected proposal */
+                    if (prepared != gcur) {
+                        nconst = grad_prepare(ws.prog[gcur], cur_ninstr, ws, lane);
+                        prepared = gcur;
+                    }
                     const float* q0 = ws.Cs[ccur];
                     float* q = ws.Cs[ccur ^ 1];
                     float k0 = 0.0f;
@@ -583,10 +867,10 @@ __global__ void __launch_bounds__(256) mh_hmc_kernel(const __grid_constant__ KPa
                         ok = __all_sync(FULLMASK, fin);
                         __syncwarp();
                         if (!ok) break;
-                        build_eval_program(ws.prog[cur], q, cur_ninstr, ws.eprog, lane);
+                        build_grad_program(ws.gprog, q, cur_ninstr, ws.eprog, lane);
                         __syncwarp();
                         int pe = 0;
-                        lik = eval_loglik_grad<K, MAXI, NV, STREAM>(ws.eprog, cur_ninstr, ws, dv, p, lane, pe, ws.gnew);
+                        lik = eval_loglik_grad<MAXR, NV, STREAM>(ws.eprog, cur_ninstr, nconst, ws, dv, p, lane, pe, ws.gnew);
                         st_pts += (unsigned)pe;
                         st_evals++; st_nodes += (unsigned)cur_count;
                         st_np += (unsigned long long)(cur_count + 4) * (unsigned)pe;
@@ -661,7 +945,7 @@ __global__ void __launch_bounds__(256) mh_hmc_kernel(const __grid_constant__ KPa
 }
 
 /* The kernels for three input variables (gpr_hmc_v.cu). */
-const void* grad_kernel_v3(int maxi, int stream);
+const void* grad_kernel_v3(int maxr, int stream);
 const void* hmc_kernel_v3(const KParams& p, int stream);
 
 }  // namespace gpr

@@ -7,23 +7,23 @@
 
 namespace gpr {
 
-const void* grad_kernel_v3(int maxi, int stream) {
-    if (maxi <= 130)
-        return stream ? (const void*)loglik_grad_kernel<GPR_HMC_K, 130, true, 3>
-                      : (const void*)loglik_grad_kernel<GPR_HMC_K, 130, false, 3>;
-    return stream ? (const void*)loglik_grad_kernel<GPR_HMC_K, 258, true, 3>
-                  : (const void*)loglik_grad_kernel<GPR_HMC_K, 258, false, 3>;
+const void* grad_kernel_v3(int maxr, int stream) {
+    if (maxr <= 96)
+        return stream ? (const void*)loglik_grad_kernel<96, true, 3>
+                      : (const void*)loglik_grad_kernel<96, false, 3>;
+    return stream ? (const void*)loglik_grad_kernel<192, true, 3>
+                  : (const void*)loglik_grad_kernel<192, false, 3>;
 }
 
-template <int MAXI, int RNG>
+template <int MAXR, int RNG>
 static const void* pick(int stream) {
-    return stream ? (const void*)mh_hmc_kernel<GPR_HMC_K, MAXI, RNG, true, 3>
-                  : (const void*)mh_hmc_kernel<GPR_HMC_K, MAXI, RNG, false, 3>;
+    return stream ? (const void*)mh_hmc_kernel<MAXR, RNG, true, 3>
+                  : (const void*)mh_hmc_kernel<MAXR, RNG, false, 3>;
 }
 
 const void* hmc_kernel_v3(const KParams& p, int stream) {
-    if (p.max_instr <= 130) return p.rng_mode ? pick<130, 1>(stream) : pick<130, 0>(stream);
-    return p.rng_mode ? pick<258, 1>(stream) : pick<258, 0>(stream);
+    if (p.max_instr <= 130) return p.rng_mode ? pick<96, 1>(stream) : pick<96, 0>(stream);
+    return p.rng_mode ? pick<192, 1>(stream) : pick<192, 0>(stream);
 }
 
 }  // namespace gpr

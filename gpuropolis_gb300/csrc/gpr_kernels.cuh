@@ -30,15 +30,16 @@ struct KParams {
     int steps;        /* MH steps this block (0 = evaluate only)             */
     uint32_t seed;    /* random_seed argument of MH_simple_kernel            */
 
-    /* dataset, staged per CTA into shared memory; arrays padded to 4 floats */
+    /* dataset, staged per CTA into shared memory; arrays in whole chunks of 128
+     * points, lane by lane (GPR_POINT_SLOT) */
     const float* dx;
     const float* dy;
     const float* dw;   /* 2^-64 / (2 sd^2) as float: weights at the bookkeeping scale */
     const float* dx2;  /* multivariate data: the second and third input variables */
     const float* dx3;
     int nv;            /* input variables: 1, or 3 for x1, x2, x3 (0 reads as 1) */
-    /* batched data (nds > 0): dataset d is points [ds_off[d], ds_off[d] + ds_n[d])
-     * of the arrays (offsets multiples of 4), with normalising sum ds_ns[2d],
+    /* batched data (nds > 0): dataset d is the ds_n[d] points from chunk ds_off[d]
+     * of the arrays on, with normalising sum ds_ns[2d],
      * ds_ns[2d+1] (2^-64 scale, double-float); chain c belongs to dataset
      * c / chains_per_ds; chain groups are claimed dataset by dataset in the
      * order ds_order (largest first); nd / nd_pad then give the largest */
@@ -49,7 +50,7 @@ struct KParams {
     const float* ds_ns;
     const int* ds_order;
     int nd;
-    int nd_pad;        /* multiple of 4                                       */
+    int nd_pad;        /* in whole chunks of 128                              */
     float normsum_hi, normsum_lo;  /* 2^-64 * sum_d 0.5*(logf(2 PIf) + 2 logf(sd_d)), double-float
                                     * (the Hamiltonian kernel's bookkeeping)  */
     /* The weights dw are 2^-e / (2 sd^2), e chosen per handle so that every

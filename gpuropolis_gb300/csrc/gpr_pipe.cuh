@@ -122,14 +122,10 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
 
     LaneData<K> ld;
     if (ONEPASS) {
-        ld.valid = 0u;
+        float x[1][K];
+        load_points<K, 1, STREAM>(dv, 0, lane, x);
 #pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const int i = lane + 32 * k;
-            const bool v = i < dv.nd;
-            ld.x[k] = v ? data_at<STREAM>(dv, DA_X1, i) : 0.0f;
-            ld.valid |= (v ? 1u : 0u) << k;
-        }
+        for (int k = 0; k < K; ++k) ld.x[k] = x[0][k];
     }
     /* Each lane's LCG jump maps (the same in every warp), read around each
      * proposal instead of held in registers. */
