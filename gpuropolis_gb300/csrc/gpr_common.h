@@ -89,20 +89,43 @@ GPR_HDI int gpr_op_class(int o) {
  * the instruction that consumes them, so the value stack is touched only
  * where both children of a binary node are subtrees. */
 typedef uint16_t gpr_word;
+/* Codes.  An odd code is a cheap binary op (sum, difference, product): the
+ * interpreter runs them all as acc = s acc + b v or acc = acc v, with s and b
+ * +1 or -1, so that telling them apart takes no branch but the one between a
+ * sum and a product.  Bit 7 of an even code: a quotient or a power; otherwise
+ * a load, a push or a unary op. */
+#define GPR_CODE_CHEAP 1u      /* sum, difference or product                    */
+#define GPR_CODE_ACCNEG 2u     /* cheap: v - acc                                */
+#define GPR_CODE_POW 2u        /* long: a power, else a quotient                */
+#define GPR_CODE_OPNEG 4u      /* cheap: acc - v                                */
+#define GPR_CODE_ACCLEFT 4u    /* long: acc is the left operand                 */
+#define GPR_CODE_MUL 8u        /* cheap: a product                              */
+#define GPR_CODE_LONG 0x80u    /* even code: quotient or power                  */
+#define GPR_CODE_SRC(code) (((code) >> 4) & 7u)
+#define GPR_CODE_IS_CONST(code) (((code) & 0x60u) == 0u)   /* binary: operand a constant or 1 */
+enum gpr_src { SRC_C = 0, SRC_ONE = 1, SRC_X = 2, SRC_POP = 3, SRC_X2 = 4, SRC_X3 = 5 };
 enum gpr_icode {
     I_END = 0,
-    I_LDX = 1, I_LDC = 2, I_LD1 = 3, I_PUSH = 4, I_LDNAN = 5, I_LDX2 = 6, I_LDX3 = 7,
-    U_INV = 8, U_LOG, U_EXP, U_SQRT, U_SIN, U_ASIN, U_COS, U_ACOS, U_TAN, U_ATAN, U_ABS,
-    I_BIN0 = 32   /* 32 + bop*16 + accleft*8 + src (3 bits) */
+    I_LDX = 2, I_LDC = 4, I_LD1 = 6, I_PUSH = 8, I_LDNAN = 10, I_LDX2 = 12, I_LDX3 = 14,
+    U_INV = 16, U_LOG = 18, U_EXP = 20, U_SQRT = 22, U_SIN = 24, U_ASIN = 26, U_COS = 28, U_ACOS = 30, U_TAN = 32,
+    U_ATAN = 34, U_ABS = 36
 };
 enum gpr_bop { BOP_ADD = 0, BOP_SUB = 1, BOP_MUL = 2, BOP_DIV = 3, BOP_POW = 4 };
-enum gpr_src { SRC_X = 0, SRC_C = 1, SRC_ONE = 2, SRC_POP = 3, SRC_X2 = 4, SRC_X3 = 5 };
 
-#define GPR_BIN(bop, accleft, src) (I_BIN0 + (bop) * 16 + (accleft) * 8 + (src))
+#define GPR_BIN(bop, accleft, src)                                                                     \
+    (((uint32_t)(src) << 4) |                                                                          \
+     ((bop) == BOP_ADD   ? GPR_CODE_CHEAP                                                              \
+      : (bop) == BOP_SUB ? (GPR_CODE_CHEAP | ((accleft) ? GPR_CODE_OPNEG : GPR_CODE_ACCNEG))           \
+      : (bop) == BOP_MUL ? (GPR_CODE_CHEAP | GPR_CODE_MUL)                                             \
+                         : (GPR_CODE_LONG | ((bop) == BOP_POW ? GPR_CODE_POW : 0u) |                   \
+                            ((accleft) ? GPR_CODE_ACCLEFT : 0u))))
 /* fields of a binary instruction code */
-#define GPR_BIN_BOP(code) (((code) - I_BIN0) >> 4)
-#define GPR_BIN_ACCLEFT(code) (((code) >> 3) & 1u)
-#define GPR_BIN_SRC(code) ((code) & 7u)
+#define GPR_IS_BIN(code) ((code) & (GPR_CODE_CHEAP | GPR_CODE_LONG))
+#define GPR_BIN_BOP(code)                                                                              \
+    (!((code) & GPR_CODE_CHEAP) ? ((code) & GPR_CODE_POW ? BOP_POW : BOP_DIV)                          \
+     : (code) & GPR_CODE_MUL    ? BOP_MUL                                                              \
+     : (code) & (GPR_CODE_ACCNEG | GPR_CODE_OPNEG) ? BOP_SUB : BOP_ADD)
+#define GPR_BIN_ACCLEFT(code) (((code) >> 2) & 1u)   /* of a difference, quotient or power */
 
 /* Counters the MH kernel accumulates (gpr_get_stats). */
 enum gpr_stat {

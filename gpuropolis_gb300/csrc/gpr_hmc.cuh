@@ -59,6 +59,11 @@ namespace gpr {
  * for one that reads a constant that constant's place among those the program
  * reads.  1 and the invalid-op marker are constants of the nodes below, which
  * no program has (PROGRAM_LENGTH <= 127). */
+#define GW_BIN 64u           /* code >= GW_BIN: GW_BIN + bop * 16 + accleft * 8 + source, else as in gpr_icode */
+#define GW_CODE(bop, left, src) (GW_BIN + (uint32_t)(bop) * 16u + (uint32_t)(left) * 8u + (uint32_t)(src))
+#define GW_BOP(code) (((code) - GW_BIN) >> 4)
+#define GW_LEFT(code) (((code) >> 3) & 1u)
+#define GW_SRC(code) ((code) & 7u)
 #define GW_ROW(w) (((w) >> 16) & 255u)
 #define GW_AUX(w) ((w) >> 24)
 #define GW_NONE 255u
@@ -146,10 +151,11 @@ static __device__ int grad_prepare(const gpr_word* prog, int ninstr, const GradS
                 code = I_LDC;
             }
             bool takes = code == I_LDC;                 /* a constant or a popped value has a share */
-            if (code >= I_BIN0) {
+            if (GPR_IS_BIN(code)) {
                 const uint32_t bop = GPR_BIN_BOP(code), left = GPR_BIN_ACCLEFT(code);
-                uint32_t src = GPR_BIN_SRC(code);
-                if (src == SRC_ONE) { src = SRC_C; node = GW_NODE_ONE; code = GPR_BIN(bop, left, SRC_C); }
+                uint32_t src = GPR_CODE_SRC(code);
+                if (src == SRC_ONE) { src = SRC_C; node = GW_NODE_ONE; }
+                code = GW_CODE(bop, left, src);
                 takes = src == SRC_POP || (src == SRC_C && node < GW_NODE_ONE);
                 if (src == SRC_POP) { --sp; aux = GW_ROW(ws.gprog[st[sp]]); }
                 if (bop == BOP_MUL) need_arg = takes;
@@ -198,38 +204,29 @@ static __device__ __noinline__ float4 pow_four(float4 u, float4 w) {
 static __device__ __noinline__ float4 log_four(float4 a) {
     return make_float4(gx_log(a.x), gx_log(a.y), gx_log(a.z), gx_log(a.w));
 }
-/* The trigonometric ops (CUDA's math library) one point after the other: each
- * round takes the first of the four values and puts its result last. */
-static __device__ __noinline__ float4 trig_four(uint32_t code, float4 a) {
-#pragma unroll 1
-    for (int n = 0; n < 4; ++n) {
-        float r;
-        switch (code) {
-            case U_SIN: r = sinf(a.x); break;
-            case U_ASIN: r = asinf(a.x); break;
-            case U_COS: r = cosf(a.x); break;
-            case U_ACOS: r = acosf(a.x); break;
-            case U_TAN: r = tanf(a.x); break;
-            default: r = atanf(a.x); break;
-        }
-        a = make_float4(a.y, a.z, a.w, r);
-    }
-    return a;
-}
-/* Their derivatives in the argument a (tan: in its result). */
+/* The derivatives of the trigonometric ops in the argument a (tan: in its
+ * result). */
 static __device__ __noinline__ float4 trig_slope_four(uint32_t code, float4 a) {
 #pragma unroll 1
-    for (int n = 0; n < 4; ++n) {
-        float r;
+    for (int n = 0; n < 2; ++n) {
+        float2 r;
         switch (code) {
-            case U_SIN: r = cosf(a.x); break;
-            case U_ASIN: r = __fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(a.x, a.x)))); break;
-            case U_COS: r = -sinf(a.x); break;
-            case U_ACOS: r = -__fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, __fmul_rn(a.x, a.x)))); break;
-            case U_TAN: r = __fadd_rn(1.0f, __fmul_rn(a.x, a.x)); break;
-            default: r = __fdiv_rn(1.0f, __fadd_rn(1.0f, __fmul_rn(a.x, a.x))); break;
+            case U_SIN: r = make_float2(cosf(a.x), cosf(a.y)); break;
+            case U_COS: r = make_float2(-sinf(a.x), -sinf(a.y)); break;
+            default: {
+                const float2 q = make_float2(__fmul_rn(a.x, a.x), __fmul_rn(a.y, a.y));
+                if (code == U_ASIN || code == U_ACOS) {
+                    r = make_float2(__fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, q.x))),
+                                    __fdiv_rn(1.0f, __fsqrt_rn(__fsub_rn(1.0f, q.y))));
+                    if (code == U_ACOS) r = make_float2(-r.x, -r.y);
+                } else {
+                    r = make_float2(__fadd_rn(1.0f, q.x), __fadd_rn(1.0f, q.y));
+                    if (code == U_ATAN) r = make_float2(__fdiv_rn(1.0f, r.x), __fdiv_rn(1.0f, r.y));
+                }
+                break;
+            }
         }
-        a = make_float4(a.y, a.z, a.w, r);
+        a = make_float4(a.z, a.w, r.x, r.y);
     }
     return a;
 }
@@ -274,7 +271,7 @@ __device__ __forceinline__ void result_of(uint32_t r, const float (&x)[NV][K], c
 template <int K, int NV>
 __device__ __forceinline__ void operand(uint32_t w, float c, const float (&x)[NV][K], const Tape<K>& tape,
                                         float (&v)[K]) {
-    const uint32_t src = GPR_BIN_SRC(w & 0xffu);
+    const uint32_t src = GW_SRC(w & 0xffu);
     if (src == SRC_C) {
 #pragma unroll
         for (int k = 0; k < K; ++k) v[k] = c;
@@ -286,8 +283,6 @@ __device__ __forceinline__ void operand(uint32_t w, float c, const float (&x)[NV
         for (int k = 0; k < K; ++k) v[k] = x[vi][k];
     }
 }
-
-#define GPR_EACH _Pragma("unroll") for (int k = 0; k < K; ++k)
 
 template <int K>
 __device__ __forceinline__ void pow_all(const float (&u)[K], const float (&w)[K], float (&r)[K]) {
@@ -331,9 +326,9 @@ __device__ __forceinline__ void forward_tape(const uint2* __restrict__ prog, int
         const uint32_t w = nxt.x, code = w & 0xffu;
         const float c = __uint_as_float(nxt.y);
         nxt = prog[i + 1];
-        if (code >= I_BIN0) {
-            const uint32_t bop = GPR_BIN_BOP(code), src = GPR_BIN_SRC(code);
-            const bool left = GPR_BIN_ACCLEFT(code);
+        if (code >= GW_BIN) {
+            const uint32_t bop = GW_BOP(code), src = GW_SRC(code);
+            const bool left = GW_LEFT(code);
             if (bop <= BOP_MUL && src == SRC_C) {
                 if (bop == BOP_ADD) { GPR_EACH acc[k] = __fadd_rn(acc[k], c); }
                 else if (bop == BOP_MUL) { GPR_EACH acc[k] = __fmul_rn(acc[k], c); }
@@ -430,9 +425,9 @@ __device__ __forceinline__ void backward_tape(const uint2* __restrict__ prog, in
         const float c = __uint_as_float(nxt.y);
         nxt = prog[i > 0 ? i - 1 : 0];
         const uint32_t arg = GW_ROW(nxt.x);       /* where the accumulator before this instruction is */
-        if (code >= I_BIN0) {
-            const uint32_t bop = GPR_BIN_BOP(code), src = GPR_BIN_SRC(code);
-            const bool left = GPR_BIN_ACCLEFT(code);
+        if (code >= GW_BIN) {
+            const uint32_t bop = GW_BOP(code), src = GW_SRC(code);
+            const bool left = GW_LEFT(code);
             if (bop == BOP_ADD) {
                 if (src == SRC_C) give_share<K>(adj, w, ws, lane);
                 else if (src == SRC_POP) tape.put(GW_AUX(w), adj);   /* the pushed value is done with */

@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
 #define ST_ADD(i, v) do { if (lane == 0) s_st[warp][(i)] += (unsigned long long)(v); } while (0)
 
     __shared__ PipeSlot s_slot[2][8];
-    __shared__ const gpr_word* s_pp[2][8];   /* published program ...          */
-    __shared__ const float* s_pc[2][8];      /* ... and its constants          */
+    __shared__ uint32_t s_pp[2][8];          /* published program (smem_offset) ... */
+    __shared__ uint32_t s_pc[2][8];          /* ... and its constants          */
     __shared__ int s_cost[2][8];             /* its length (-1: none)          */
     __shared__ int s_cnt[2][8];              /* its node count                 */
     __shared__ int s_bad[2][8];              /* a point was invalid            */
@@ -360,8 +360,8 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                     s_cost[g][warp] = publish;
                     s_cnt[g][warp] = count;
                     s_bad[g][warp] = 0;
-                    s_pp[g][warp] = wg.prog[gbuf & 1];
-                    s_pc[g][warp] = wg.Cs[cbuf & 1];
+                    s_pp[g][warp] = smem_offset(wg.prog[gbuf & 1]);
+                    s_pc[g][warp] = smem_offset(wg.Cs[cbuf & 1]);
                 }
                 __syncwarp();
             }
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                     const int piece = t - q * tpc;
                     const int w = __ffs(__ballot_sync(FULLMASK, my_rank == q)) - 1;
                     if (s_bad[e][w]) continue;
-                    const PCProg prog = {s_pp[e][w], s_pc[e][w]};
+                    const PCProg prog = {(const gpr_word*)(gpr_dyn_smem + s_pp[e][w]), (const float*)(gpr_dyn_smem + s_pc[e][w])};
                     float* pr = part_row(e, w);
                     const int p0 = piece * ppt, p1 = min(npass, p0 + ppt);
                     int np = 0;
