@@ -397,7 +397,7 @@ static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int s
     if (!gpr::grad_supported(kp))
         return fail(h, GPR_ERR_ARG, "gradient moves support program_length <= 127 (got %d)", kp.PL);
     gpr::LaunchCfg lc;
-    lc.K = 4; lc.onepass = 0; lc.rolled = 0; lc.lockstep = 0; lc.carveout = 0;
+    lc.K = 4; lc.onepass = 0; lc.rolled = 0; lc.lockstep = 0; lc.carveout = 0; lc.pipe = 0;
     /* Streamed when asked, for batched data (each warp reads its own chain's
      * dataset from device memory), when staging does not fit, and when the
      * staged copy would take over a quarter of the CTA's shared memory: the
@@ -431,8 +431,8 @@ static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int s
     return GPR_OK;
 }
 
-/* A dataset is streamed from device memory when the caller asks for it, or
- * when staging it beside a full CTA of warps would not fit in shared memory;
+/* A dataset is streamed from device memory when the caller asks for it (or
+ * choose_launch does), or when staging it beside a full CTA of warps would not fit in shared memory;
  * streaming uses K = 4 points per lane in passes.  pipe: the pipelined kernel
  * (two chains per warp, one barrier per half-step; lockstep is then unused);
  * it needs heavy ops unrolled, and for batched data chain groups of
@@ -504,15 +504,31 @@ static int configure_launch(gpr_handle* h, int K, int onepass, int rolled, int l
 }
 
 /* Default layout before any autotuning: K = 4 points per lane, one pass when
- * the data fit, heavy ops unrolled; the lockstep kernel while a CTA can
+ * the data fit, heavy ops in registers; the lockstep kernel while a CTA can
  * balance its chains' passes over its warps (up to GPR_MAX_PASSES passes: on
  * the 250-point workload it measured 10% faster), the pipelined kernel beyond
  * (which splits any number of passes over the warps: 20% faster on the
  * 65,536-point workload than free-running warps).  Three input variables and
- * batched data take K = 4 in passes (gpr_autotune re-checks per dataset). */
+ * batched data take K = 4 in passes (gpr_autotune re-checks per dataset).
+ *
+ * The data are streamed where staging them would leave fewer of the chains'
+ * CTAs resident: they stay in L1 and L2, and the kernels, bound by latency and
+ * instruction fetch, need the warps.  256 datasets of up to 4,096 points, PL 47
+ * (2 CTAs per SM staged, 3 streamed): 206 -> 157 ms; 131,072 programs scored on
+ * 4,096 points, PL 31 (2, 3): 3.47 -> 2.79 ms; 1,501 points, PL 127 (2, 3): 14.3
+ * -> 13.6 ms.  With as many either way, both take the same time (250 points,
+ * PL 63: 185.7 and 186.3 ms; 500 points, PL 31: 41.2 and 41.3 ms). */
 static int choose_launch(gpr_handle* h) {
     const int pipe = (h->kp.nd + 127) / 128 > GPR_MAX_PASSES ? 1 : 0;
-    return configure_launch(h, 4, (h->kp.nd <= 128 && h->kp.nv != 3 && h->kp.nds == 0) ? 1 : 0, 0, 1, 8, pipe);
+    const int onepass = (h->kp.nd <= 128 && h->kp.nv != 3 && h->kp.nds == 0) ? 1 : 0;
+    int rc = configure_launch(h, 4, onepass, 0, 1, 8, pipe);
+    if (rc != GPR_OK || h->kp.const_mode == GPR_CONST_HMC || h->lc.stream || onepass || h->kp.nd <= 0) return rc;
+    const int staged = h->lc.ctas;
+    h->stream_data = 1;
+    rc = configure_launch(h, 4, 0, 0, 1, 8, pipe);
+    h->stream_data = 0;
+    if (rc == GPR_OK && h->lc.ctas > staged) return rc;
+    return configure_launch(h, 4, 0, 0, 1, 8, pipe);
 }
 
 /* Device layout of a dataset: x1 | y | w | sd | x2 | x3, nd_pad floats each

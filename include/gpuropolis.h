@@ -211,7 +211,8 @@ int gpr_set_layout3(gpr_handle* h, int K, int onepass, int rolled, int lockstep,
 
 /* Read the dataset from device memory in every pass (always = 1) instead of
  * staging it into each CTA's shared memory; 0 (default) streams only when
- * staging does not fit, as for datasets of tens of thousands of points.
+ * staging does not fit, as for datasets of tens of thousands of points, or
+ * would keep fewer of the chains resident at once.
  * Results are identical either way.  gpr_layout_streamed reports the mode
  * of the current layout. */
 int gpr_set_streaming(gpr_handle* h, int always);
