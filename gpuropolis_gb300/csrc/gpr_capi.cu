@@ -454,10 +454,13 @@ static int configure_launch(gpr_handle* h, int K, int onepass, int rolled, int l
         wpc0 = batched_wpc(kp, wpc0, pipe);
     }
     auto smem_of = [&](int k, int w, int st) {
-        return pipe ? gpr::pipe_smem_bytes(kp, k, w, st) : gpr::mh_smem_bytes(kp, k, w, st);
+        return pipe ? gpr::pipe_smem_bytes(kp, k, w, st) : gpr::mh_smem_bytes(kp, k, w, st, rolled);
     };
     lc.stream = h->stream_data || smem_of(K, wpc0, 0) > 227 * 1024;
-    if (lc.stream) { K = 4; onepass = 0; }
+    if (lc.stream) {
+        if (kp.nds > 0 || rolled) K = 4;
+        onepass = 0;
+    }
     lc.K = K;
     lc.onepass = onepass;
     lc.rolled = rolled;
@@ -482,12 +485,15 @@ static int configure_launch(gpr_handle* h, int K, int onepass, int rolled, int l
     long long need = (h->N + per_cta - 1) / per_cta;
     if (ctas > need) ctas = need;
     lc.ctas = (int)ctas;
-    /* chunk sums beyond the pipelined kernel's shared-memory board: one row
-     * per (CTA, group, warp) in device memory */
+    /* chunk sums beyond the kernel's shared-memory board: one row per chain in
+     * flight (8 per CTA, 16 of the pipelined kernel) in device memory */
     kp.part_stride = 0;
-    const int stride = pipe ? gpr::pipe_part_stride(kp.nd) : 0;
+    const bool many = !pipe && lc.K == 8 && lc.stream;
+    const int passes = (kp.nd + 32 * lc.K - 1) / (32 * lc.K);
+    kp.ppt = std::max(1, (passes + GPR_TASKS - 1) / GPR_TASKS);
+    const int stride = pipe ? gpr::pipe_part_stride(kp.nd) : many ? gpr::mh_part_stride(kp.nd) : 0;
     if (stride > 0) {
-        const size_t need_f = (size_t)lc.ctas * 16 * (size_t)stride;
+        const size_t need_f = (size_t)lc.ctas * (pipe ? 16 : 8) * (size_t)stride;
         if (h->dpart_floats < need_f) {
             CUDA_TRY(h, cudaStreamSynchronize(h->stream));
             cudaFree(h->dpart);
@@ -503,30 +509,53 @@ static int configure_launch(gpr_handle* h, int K, int onepass, int rolled, int l
     return GPR_OK;
 }
 
-/* Default layout before any autotuning: K = 4 points per lane, one pass when
- * the data fit, heavy ops in registers; the lockstep kernel while a CTA can
- * balance its chains' passes over its warps (up to GPR_MAX_PASSES passes: on
- * the 250-point workload it measured 10% faster), the pipelined kernel beyond
- * (which splits any number of passes over the warps: 20% faster on the
- * 65,536-point workload than free-running warps).  Three input variables and
- * batched data take K = 4 in passes (gpr_autotune re-checks per dataset).
- *
- * The data are streamed where staging them would leave fewer of the chains'
- * CTAs resident: they stay in L1 and L2, and the kernels, bound by latency and
- * instruction fetch, need the warps.  256 datasets of up to 4,096 points, PL 47
- * (2 CTAs per SM staged, 3 streamed): 206 -> 157 ms; 131,072 programs scored on
- * 4,096 points, PL 31 (2, 3): 3.47 -> 2.79 ms; 1,501 points, PL 127 (2, 3): 14.3
- * -> 13.6 ms.  With as many either way, both take the same time (250 points,
- * PL 63: 185.7 and 186.3 ms; 500 points, PL 31: 41.2 and 41.3 ms). */
-static int choose_launch(gpr_handle* h) {
-    const int pipe = (h->kp.nd + 127) / 128 > GPR_MAX_PASSES ? 1 : 0;
-    const int onepass = (h->kp.nd <= 128 && h->kp.nv != 3 && h->kp.nds == 0) ? 1 : 0;
-    int rc = configure_launch(h, 4, onepass, 0, 1, 8, pipe);
-    if (rc != GPR_OK || h->kp.const_mode == GPR_CONST_HMC || h->lc.stream || onepass || h->kp.nd <= 0) return rc;
-    const int staged = h->lc.ctas;
+/* A launch that streams the data, whatever the caller asked for. */
+static int configure_streamed(gpr_handle* h, int K, int pipe) {
+    const int asked = h->stream_data;
     h->stream_data = 1;
-    rc = configure_launch(h, 4, 0, 0, 1, 8, pipe);
-    h->stream_data = 0;
+    const int rc = configure_launch(h, K, 0, 0, 1, 8, pipe);
+    h->stream_data = asked;
+    return rc;
+}
+
+/* Passes (of 128 points) from which the default layout takes K = 8: with one
+ * input variable, with three. */
+#define GPR_MANY_PASSES 32
+#define GPR_MANY_PASSES3 48
+
+/* Default layout before any autotuning: the lockstep kernel, heavy ops in
+ * registers, K = 4 points per lane, in one pass when the data fit.
+ *
+ * From GPR_MANY_PASSES passes on: streamed, with K = 8, a task being a range of
+ * passes.  An instruction is then decoded once for two passes of 128 points,
+ * and there are tasks enough that coarser ones still balance.  16,384 chains,
+ * 20 steps, K = 4 / K = 8: 2,048 points 5.86 / 5.83 ms (basic ops, PL 63) and
+ * 4.66 / 5.09 (all ops, PL 31); 4,096 points 10.0 / 9.2 and 8.19 / 8.11; 8,000
+ * points 17.7 / 16.1 and 14.2 / 13.7; three variables, 8,192 chains, 40 steps:
+ * 4,100 points 7.18 / 7.55, 8,000 points 13.4 / 12.5.  Beyond 64 passes, where K = 4 leaves each
+ * warp its own chain: 65,536 points of three variables, PL 127: 240 / 65 ms,
+ * and 79 ms for the pipelined kernel with K = 8, which spreads a chain's passes
+ * too but interprets programs in place.  Batched data (groups of uneven
+ * datasets) of more than 64 passes go to the pipelined kernel.
+ *
+ * Fewer passes: staged, unless that would leave fewer of the chains' CTAs
+ * resident.  Streamed data stay in L1 and L2, and the kernels, bound by latency
+ * and instruction fetch, need the warps.  256 datasets of up to 4,096 points,
+ * PL 47 (2 CTAs per SM staged, 3 streamed): 206 -> 157 ms; 1,501 points, PL 127
+ * (2, 3): 14.3 -> 13.6 ms.  With as many either way, both take the same time
+ * (250 points, PL 63: 185.7 and 186.3 ms; 500 points, PL 31: 41.2 and 41.3). */
+static int choose_launch(gpr_handle* h) {
+    const gpr::KParams& kp = h->kp;
+    const int passes = (kp.nd + 127) / 128;
+    const int pipe = kp.nds > 0 && passes > GPR_MAX_PASSES ? 1 : 0;
+    const int onepass = (kp.nd <= 128 && kp.nv != 3 && kp.nds == 0) ? 1 : 0;
+    const bool hmc = kp.const_mode == GPR_CONST_HMC;
+    if (!hmc && kp.nds == 0 && passes >= (kp.nv == 3 ? GPR_MANY_PASSES3 : GPR_MANY_PASSES))
+        return configure_streamed(h, 8, 0);
+    int rc = configure_launch(h, 4, onepass, 0, 1, 8, pipe);
+    if (rc != GPR_OK || hmc || h->lc.stream || onepass || kp.nd <= 0) return rc;
+    const int staged = h->lc.ctas;
+    rc = configure_streamed(h, 4, pipe);
     if (rc == GPR_OK && h->lc.ctas > staged) return rc;
     return configure_launch(h, 4, 0, 0, 1, 8, pipe);
 }

@@ -167,9 +167,12 @@ enum gpr_phase {
     GPR_PH_SLOTS
 };
 
-/* Passes (32*K points each) a CTA-balanced evaluation can split a dataset
- * into; beyond it each warp evaluates its own chain. */
+/* Passes (32*K points each) that the lockstep kernel splits a chain's
+ * evaluation into, one task each; with K = 8 streamed a task is a range of
+ * passes, GPR_TASKS of them per chain at most, and the sums of more than
+ * GPR_MAX_PASSES chunks are kept in device memory (KParams::part). */
 #define GPR_MAX_PASSES 64
+#define GPR_TASKS 16
 
 /* ---- dataset arrays ----
  * Points are kept in chunks of 128, the unit of the likelihood's reduction

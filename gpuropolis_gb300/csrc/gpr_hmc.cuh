@@ -258,8 +258,7 @@ __device__ __forceinline__ void result_of(uint32_t r, const float (&x)[NV][K], c
         tape.get(r, v);
     } else {
         const int vi = NV > 1 ? (int)(GW_X1 - r) : 0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = x[vi][k];
+        GPR_EACH v[k] = x[vi][k];
     }
 }
 
@@ -276,8 +275,7 @@ __device__ __forceinline__ void operand(uint32_t w, float c, const float (&x)[NV
         tape.get(GW_AUX(w), v);
     } else {
         const int vi = NV > 1 && src != SRC_X ? (int)(src - SRC_X2) + 1 : 0;
-#pragma unroll
-        for (int k = 0; k < K; ++k) v[k] = x[vi][k];
+        GPR_EACH v[k] = x[vi][k];
     }
 }
 
@@ -371,8 +369,7 @@ __device__ __forceinline__ void forward_tape(const uint2* __restrict__ prog, int
             for (int k = 0; k < K; ++k) acc[k] = c;
         } else if (code != I_PUSH) {
             const int vi = NV > 1 && code != I_LDX ? (code == I_LDX2 ? 1 : 2) : 0;
-#pragma unroll
-            for (int k = 0; k < K; ++k) acc[k] = x[vi][k];
+            GPR_EACH acc[k] = x[vi][k];
         }
         const uint32_t row = GW_ROW(w);
         if (row < GW_X3) tape.put(row, acc);

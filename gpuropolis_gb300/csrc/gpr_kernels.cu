@@ -8,9 +8,14 @@
 namespace gpr {
 
 /* ------------------------------------------------------------------------ */
-size_t mh_smem_bytes(const KParams& p, int K, int warps_per_cta, int stream) {
+size_t mh_smem_bytes(const KParams& p, int K, int warps_per_cta, int stream, int rolled) {
     return 16 + (stream ? 0 : align16((size_t)data_arrays(p) * p.nd_pad * 4)) +
-           (size_t)warps_per_cta * warp_smem_bytes(p.PL, p.max_instr, p.levels, K);
+           (size_t)warps_per_cta * warp_smem_bytes(p.PL, p.max_instr, p.levels, K, rolled != 0);
+}
+
+int mh_part_stride(int nd) {
+    const int nch = (nd + GPR_CHUNK_POINTS - 1) / GPR_CHUNK_POINTS;
+    return nch <= GPR_MAX_PASSES ? 0 : nch;
 }
 
 int pipe_part_stride(int nd) {
@@ -26,6 +31,7 @@ size_t pipe_smem_bytes(const KParams& p, int K, int warps_per_cta, int stream) {
 
 static const void* pick_pipe(int K, int onepass, int rng, int rolled, int stream, int nv, int batched) {
     if (batched) return (K == 4 && !onepass) ? pipe_kernel_k4b(rng, rolled, stream, nv) : nullptr;
+    if (K == 8 && stream) return (rolled || onepass) ? nullptr : pipe_kernel_k8s(rng, nv);
     if (nv == 3) return (K == 4 && !onepass) ? pipe_kernel_k4v(rng, rolled, stream) : nullptr;
     if (K == 4) return pipe_kernel_k4(rng, rolled, onepass, stream);
     if (K == 8) return stream ? nullptr : pipe_kernel_k8(rng, rolled, onepass);
@@ -38,6 +44,7 @@ static const void* pick_kernel(int K, int onepass, int rng, int rolled, int stre
         if (K != 4 || onepass) return nullptr;
         return nv == 3 ? mh_kernel_k4bv(rng, rolled, stream) : mh_kernel_k4b(rng, rolled, stream);
     }
+    if (stream && K == 8) return (rolled || onepass) ? nullptr : mh_kernel_k8s(rng, nv);
     if (nv == 3) return (K == 4 && !onepass) ? mh_kernel_k4v(rng, rolled, stream) : nullptr;
     if (stream) return (K == 4 && !onepass) ? mh_kernel_k4s(rng, rolled) : nullptr;
     if (K == 4) return onepass ? mh_kernel_k4(rng, rolled) : mh_kernel_k4m(rng, rolled);
@@ -81,7 +88,7 @@ __global__ void __launch_bounds__(128) eval_values_kernel(const __grid_constant_
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    const size_t wbytes = warp_smem_bytes(p.PL, p.max_instr, p.levels, 1);
+    const size_t wbytes = warp_smem_bytes(p.PL, p.max_instr, p.levels, 1, false);
     WarpSmem ws = carve_warp<1>(smem + (size_t)warp * wbytes, p.PL, p.max_instr, p.levels);
     const int chain = blockIdx.x * (blockDim.x >> 5) + warp;
     if (chain >= p.N) return;
@@ -114,7 +121,7 @@ __global__ void __launch_bounds__(128) eval_values_kernel(const __grid_constant_
 cudaError_t launch_eval_values(const KParams& p, const float* xs, int nx, float* out,
                                float* length, int* count, cudaStream_t st) {
     const int wpc = 4;
-    size_t smem = (size_t)wpc * warp_smem_bytes(p.PL, p.max_instr, p.levels, 1);
+    size_t smem = (size_t)wpc * warp_smem_bytes(p.PL, p.max_instr, p.levels, 1, false);
     cudaError_t e = cudaFuncSetAttribute((const void*)eval_values_kernel,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -67,9 +67,12 @@ struct KParams {
     float ln1u_hi, ln1u_lo; /* log((double)NOPS + 1) as a double-float (main.cu:536) */
     float cauchy_c_hi, cauchy_c_lo;   /* PL * logf(PIf), the constant part of the
                                        * Cauchy prior (main.cu:304, 537-540), double-float */
-    float* part;            /* chunk sums of the pipelined kernel when a dataset has more
-                             * chunks than its shared-memory board holds      */
-    int part_stride;        /* floats per (CTA, group, warp) in part          */
+    float* part;            /* chunk sums when a dataset has more chunks than the
+                             * kernel's shared-memory board holds              */
+    int part_stride;        /* floats per chain in flight in part: per (CTA, warp),
+                             * for the pipelined kernel per (CTA, group, warp) */
+
+    int ppt;                /* passes per task of the lockstep kernel with K = 8 streamed */
 
     /* proposals */
     int rng_mode;      /* 0 LCG, 1 Philox                                     */
@@ -99,7 +102,7 @@ struct KParams {
     int lockstep;      /* >0: the warps of a CTA realign every `lockstep` steps  */
     int stage_wait_iters;  /* polls of the dataset staging barrier before the kernel
                             * gives up with error flag 1 (default 2^22)          */
-    int levels;        /* value-stack slots per lane                            */
+    int levels;        /* value-stack depth: pushes pending at most             */
     int max_instr;     /* instruction buffer length per program                 */
 
     /* move schedule and Hamiltonian constant moves */
@@ -133,6 +136,7 @@ const void* mh_kernel_k4(int rng, int rolled);
 const void* mh_kernel_k4m(int rng, int rolled);
 const void* mh_kernel_k8(int rng, int rolled);
 const void* mh_kernel_k8m(int rng, int rolled);
+const void* mh_kernel_k8s(int rng, int nv);   /* the same, K = 8 */
 const void* mh_kernel_k4s(int rng, int rolled);   /* dataset streamed from device memory */
 const void* mh_kernel_k4v(int rng, int rolled, int stream);   /* three input variables */
 const void* mh_kernel_k4b(int rng, int rolled, int stream);    /* batched data */
@@ -152,13 +156,15 @@ struct LaunchCfg {
     int stream;        /* dataset read from device memory, not staged per CTA   */
 };
 
-size_t mh_smem_bytes(const KParams& p, int K, int warps_per_cta, int stream = 0);
+size_t mh_smem_bytes(const KParams& p, int K, int warps_per_cta, int stream, int rolled);
 size_t pipe_smem_bytes(const KParams& p, int K, int warps_per_cta, int stream = 0);
 /* Chunk-sum floats the pipelined kernel needs in p.part for nd points (0:
  * its shared-memory board suffices), per (CTA, group, warp). */
 int pipe_part_stride(int nd);
+int mh_part_stride(int nd);   /* the same for the lockstep kernel, per (CTA, warp) */
 const void* pipe_kernel_k4(int rng, int rolled, int onepass, int stream);
 const void* pipe_kernel_k8(int rng, int rolled, int onepass);
+const void* pipe_kernel_k8s(int rng, int nv);   /* large streamed data */
 const void* pipe_kernel_k4v(int rng, int rolled, int stream);
 const void* pipe_kernel_k4b(int rng, int rolled, int stream, int nv);
 cudaError_t launch_mh_block(const KParams& p, const LaunchCfg& lc, cudaStream_t st);

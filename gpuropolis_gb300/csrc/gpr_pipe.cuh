@@ -53,14 +53,14 @@ struct PipeSlot {
 
 /* Per-warp dynamic shared memory: per slot the op, constant and program
  * buffers (current and proposal), then one region shared by the slots' turns
- * and the warp's evaluation tasks (value stack and transcendental scratch |
- * constant-move records | compiler scratch). */
+ * and the warp's evaluation tasks (value stack | constant-move records |
+ * compiler scratch). */
 __host__ __device__ __forceinline__ size_t pipe_slot_bytes(int PL, int max_instr) {
     const size_t plp = align16((size_t)PL);
     return 2 * plp + align16(2 * plp * 4) + align16(2 * (size_t)max_instr * sizeof(gpr_word));
 }
 __host__ __device__ __forceinline__ size_t pipe_warp_bytes(int PL, int max_instr, int levels, int K) {
-    return 2 * pipe_slot_bytes(PL, max_instr) + shared_region_bytes(PL, levels, K);
+    return 2 * pipe_slot_bytes(PL, max_instr) + shared_region_bytes(PL, levels, K, false);
 }
 
 /* The CTA's chunk-sum board, [2 groups][8 warps][GPR_PIPE_CHUNKS] floats, in
@@ -82,7 +82,7 @@ __device__ __forceinline__ WarpSmem carve_pipe(uint8_t* base, int PL, int max_in
     w.eprog = nullptr;
     uint8_t* r = base + 2 * pipe_slot_bytes(PL, max_instr);
     w.stk = (float*)r;
-    w.scr = w.stk + (size_t)levels * K * 32;
+    w.scr = nullptr;   /* heavy ops in registers only */
     w.off = (int*)r;
     w.ndr = w.off + plp;
     w.fw = (float*)(w.ndr + plp);
@@ -116,9 +116,8 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
     }
     const int PL = p.PL;
     uint8_t* const mybase = wbase + (size_t)warp * pipe_warp_bytes(PL, p.max_instr, p.levels, K);
-    /* the warp's value stack and transcendental scratch for its evaluation tasks */
+    /* the warp's value stack for its evaluation tasks */
     float* const my_stk = (float*)(mybase + 2 * pipe_slot_bytes(PL, p.max_instr));
-    float* const my_scr = my_stk + (size_t)p.levels * K * 32;
 
     LaneData<K> ld;
     if (ONEPASS) {
@@ -400,7 +399,7 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
 #pragma unroll 1
                     for (int pass = p0; pass < p1; ++pass) {
                         float csum[K / 4];
-                        const bool bad = eval_pass_chunks<K, ONEPASS, ROLLED, NV, STREAM>(prog, my_stk, my_scr, ld,
+                        const bool bad = eval_pass_chunks<K, ONEPASS, ROLLED, NV, STREAM>(prog, my_stk, nullptr, ld,
                                                                                         dv, p, lane, pass, csum);
                         np += ONEPASS ? dv.nd : min(32 * K, dv.nd - pass * 32 * K);
                         if (lane == 0) {
