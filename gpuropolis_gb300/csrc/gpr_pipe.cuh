@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                         } else if (!init) {
                             /* ---- constant move (main.cu:743-806) ---- */
                             df fws, bws;
-                            constant_move<RNG>(r, wg, wg.Cs[ccur], wg.Cs[ccur ^ 1], fws, bws, cs, p, s_lj[lane], lane, rw_sd);
+                            constant_move<RNG>(r, wg, wg.Cs[ccur], wg.Cs[ccur ^ 1], fws, bws, p, s_lj[lane], lane, rw_sd);
                             if (p.const_mode == 0) { fw = df_add(fw, fws); bw = df_add(bw, bws); }
                             pbuf = cur; cbuf = ccur ^ 1; gbuf = gcur;
                             len = cur_len; count = cur_count; ninstr = cur_ninstr; reads = cur_reads;
@@ -322,8 +322,7 @@ __global__ void __launch_bounds__(256, GPR_MIN_CTAS) mh_pipe_kernel(const __grid
                             bw = df_make(-p.logcount[count], 0.0f);
                             cs = cur_cs;
                         } else {
-                            if (init) cs = cauchy_lane(wg.Cs[cbuf], p, lane);
-                            cs = cauchy_total(cs, p);
+                            cs = cauchy_sum_u(wg.Cs[cbuf], p, lane);
                             GPR_PH(GPR_PH_CAUCHY);
                         }
                         prior = prior_u(len, cs, p);

@@ -386,8 +386,10 @@ __global__ void __launch_bounds__(GPR_RD_THREADS) redraw_kernel(const __grid_con
         const uint32_t w = s_draw[c * GPR_RD_CHAINS];
         int qu = c + 1, qv = c + 2;
         if (GPR_RD_STEP(w) == GPR_RD_FAR) { qu = find(s_unbit, qu, ~0u); qv = find(s_unbit, qu + 1, ~0u); }
-        const float z = box_muller((int)GPR_RD_UNIFORM(s_draw[qu * GPR_RD_CHAINS]),
-                                   (int)GPR_RD_UNIFORM(s_draw[qv * GPR_RD_CHAINS]));
+        const float u = gpr_rng_k_over_1e6((int)GPR_RD_UNIFORM(s_draw[qu * GPR_RD_CHAINS]));
+        const float v = gpr_rng_k_over_1e6((int)GPR_RD_UNIFORM(s_draw[qv * GPR_RD_CHAINS]));
+        const float a = __fsqrt_rn(__fmul_rn(-2.0f, gpr_rng_logf(u)));
+        const float z = __fmul_rn(a, gpr_rng_sinf(gpr_rng_twopi_times(v)));
         p.C[(size_t)i * N + chain] = __fmul_rn(s_pow10[GPR_RD_ORDER(w)], z);
     }
     if (warp == 0 && live && !fast) {
