@@ -52,6 +52,7 @@ struct gpr_handle {
     /* selection scratch, allocated by the first gpr_resample/gpr_top_chains/gpr_map_chain */
     float* dscale = nullptr;               /* per-chain proposal scales          */
     float* dpart = nullptr;                /* chunk sums of the pipelined kernel for large datasets */
+    double* dgrad = nullptr;               /* results of gpr_loglik_grad (N * PL + N), kept when small */
     size_t dpart_floats = 0;
     double* dds_ns64 = nullptr;            /* batched data: unscaled normalising sums */
     int stream_data = 0;                   /* 1: always stream the dataset       */
@@ -206,6 +207,7 @@ static void free_all(gpr_handle* h) {
     cudaFreeHost(h->hsel);
     cudaFree(h->dkeys); cudaFree(h->dsel); cudaFree(h->dseli); cudaFree(h->dtop); cudaFree(h->dscale);
     cudaFree(h->dds); cudaFree(h->dds_ns); cudaFree(h->dds_ns64); cudaFree(h->dpart);
+    cudaFree(h->dgrad);
     if (h->graph) cudaGraphExecDestroy(h->graph);
     if (h->graph_src) cudaGraphDestroy(h->graph_src);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
@@ -1299,6 +1301,13 @@ int gpr_chain_scales(gpr_handle* h, float* out) {
     return GPR_OK;
 }
 
+/* Results of gpr_loglik_grad up to this size stay allocated with the handle: an
+ * optimiser calls it once an iteration, and cudaMalloc with cudaFree (which waits for
+ * the device) took 0.14 of the 1.29 ms of 65,536 chains of 31 nodes on 1,024 points.
+ * Larger ones, where the copy back hides that, are given back, so that a huge
+ * population holds no more device memory between calls than its state. */
+#define GPR_GRAD_KEEP_BYTES ((size_t)256 << 20)
+
 int gpr_loglik_grad(gpr_handle* h, double* grad, double* likelihood) {
     if (!h) return GPR_ERR_ARG;
     if (!grad) return fail(h, GPR_ERR_ARG, "grad is NULL");
@@ -1307,11 +1316,13 @@ int gpr_loglik_grad(gpr_handle* h, double* grad, double* likelihood) {
         return fail(h, GPR_ERR_ARG, "gradients support program_length <= 127 (got %d)", h->PL);
 
     CUDA_TRY(h, cudaSetDevice(h->device));
-    const size_t cnt = (size_t)h->N * h->PL;
-    double* dg = nullptr;
-    double* dl = nullptr;
-    cudaError_t e = cudaMalloc(&dg, cnt * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&dl, (size_t)h->N * sizeof(double));
+    const size_t cnt = (size_t)h->N * h->PL, total = cnt + (size_t)h->N;
+    const bool keep = total * sizeof(double) <= GPR_GRAD_KEEP_BYTES;
+    double* buf = keep ? h->dgrad : nullptr;
+    cudaError_t e = buf ? cudaSuccess : cudaMalloc(&buf, total * sizeof(double));
+    if (keep && e == cudaSuccess) h->dgrad = buf;
+    double* dg = buf;
+    double* dl = e == cudaSuccess ? buf + cnt : nullptr;
     /* batched data: every warp reads its chain's dataset from device memory */
     const bool st = h->stream_data || h->kp.nds > 0 || gpr::grad_smem_bytes(h->kp, 4) > 227 * 1024;
     if (e == cudaSuccess) e = gpr::launch_loglik_grad(h->kp, dg, dl, st, h->stream);
@@ -1322,8 +1333,7 @@ int gpr_loglik_grad(gpr_handle* h, double* grad, double* likelihood) {
     if (e == cudaSuccess && likelihood)
         e = cudaMemcpyAsync(likelihood, dl, (size_t)h->N * sizeof(double), cudaMemcpyDeviceToHost, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-    cudaFree(dg);
-    cudaFree(dl);
+    if (!keep) cudaFree(buf);
     if (e != cudaSuccess) return fail(h, GPR_ERR_CUDA, "gpr_loglik_grad: %s", cudaGetErrorString(e));
     return gpr_sync(h);
 }
