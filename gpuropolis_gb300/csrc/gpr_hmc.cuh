@@ -307,6 +307,32 @@ __device__ __forceinline__ void trig_all(uint32_t code, const float (&a)[K], flo
     }
 }
 
+/* acc = acc / v, and acc = 1 / acc, with one range check for this lane's K
+ * values, where __fdiv_rn checks and branches for each.  65,536 chains of the
+ * rational function on 1,024 points, 10 moves of 8 leapfrog steps: 75.9 -> 69.6
+ * ms, their gradients 1.14 -> 1.07 ms; 2,048 programs of three variables on
+ * 16,384 points the same within the runs.  The interpreter keeps __fdiv_rn,
+ * whose code is smaller: with these 131,072 chains of 63 nodes took 208 ms
+ * instead of 199, 16,384 chains on 65,536 points 74.7 instead of 65.5. */
+template <int K>
+__device__ __forceinline__ void divide(float (&acc)[K], float (&v)[K]) {
+    if (gx_in_range(acc) && gx_in_range(v)) {
+        GPR_EACH acc[k] = gx_quotient(acc[k], v[k], gx_recip(v[k]));
+    } else {
+        in_turn<K, 1>(acc, v, [](float a, float b) { return __fdiv_rn(a, b); });
+    }
+}
+template <int K>
+__device__ __forceinline__ void invert(float (&acc)[K]) {
+    if (gx_in_range(acc)) {
+        GPR_EACH acc[k] = gx_recip(acc[k]);
+    } else {
+        float v[K];
+        GPR_EACH v[k] = 0.0f;
+        in_turn<K, 1>(acc, v, [](float a, float) { return __fdiv_rn(1.0f, a); });
+    }
+}
+
 /* acc = f(x) for this lane's K points, the results that the way back needs
  * kept on the tape.  The arithmetic is the evaluator's (run_program),
  * operation for operation. */
@@ -342,7 +368,7 @@ __device__ __forceinline__ void forward_tape(const uint2* __restrict__ prog, int
                 else {
                     if (!left) { GPR_EACH { const float t = acc[k]; acc[k] = v[k]; v[k] = t; } }
                     if (bop == BOP_SUB) { GPR_EACH acc[k] = __fsub_rn(acc[k], v[k]); }
-                    else if (bop == BOP_DIV) { GPR_EACH acc[k] = __fdiv_rn(acc[k], v[k]); }
+                    else if (bop == BOP_DIV) divide<K>(acc, v);
                     else pow_all<K>(acc, v, acc);
                 }
             }
@@ -353,8 +379,7 @@ __device__ __forceinline__ void forward_tape(const uint2* __restrict__ prog, int
             } else if (code == U_LOG) {
                 log_all<K>(acc, acc);
             } else if (code == U_INV) {
-#pragma unroll
-                for (int k = 0; k < K; ++k) acc[k] = __fdiv_rn(1.0f, acc[k]);
+                invert<K>(acc);
             } else if (code == U_SQRT) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) acc[k] = __fsqrt_rn(acc[k]);
@@ -406,6 +431,19 @@ __device__ __forceinline__ void give_share(const float (&av)[K], uint32_t w, con
             if (lane == 0) ws.gacc[(w >> 8) & 0xffu] += tot;
         }
     }
+}
+
+/* du = 1 / v, dw = -res / v for arguments out of the fast quotient's range. */
+template <int K>
+__device__ __forceinline__ void general_slopes(const float (&res)[K], const float (&v)[K], float (&du)[K],
+                                               float (&dw)[K], bool w_too) {
+    float b[K], t[K];
+    GPR_EACH { b[k] = v[k]; du[k] = 1.0f; }
+    in_turn<K, 1>(du, b, [](float a, float c) { return __fdiv_rn(a, c); });
+    if (!w_too) return;
+    GPR_EACH { b[k] = v[k]; t[k] = res[k]; }
+    in_turn<K, 1>(t, b, [](float a, float c) { return __fdiv_rn(a, c); });
+    GPR_EACH dw[k] = -t[k];
 }
 
 /* The backward sweep: adj holds d loglik / d f per point on entry. */
@@ -460,11 +498,16 @@ __device__ __forceinline__ void backward_tape(const uint2* __restrict__ prog, in
                     if (arg != GW_NONE) result_of<K, NV>(arg, x, tape, a);
                     if (GW_ROW(w) < GW_X3) tape.get(GW_ROW(w), res);
                     if (bop == BOP_DIV) {
-                        /* u / w: du = 1 / w, dw = -res / w */
+                        /* u / w: du = 1 / w, dw = -res / w, from one reciprocal */
                         if (!left) { GPR_EACH v[k] = a[k]; }
                         float du[K], dw[K];
-                        if (left || takes) { GPR_EACH du[k] = __fdiv_rn(1.0f, v[k]); }
-                        if (!left || takes) { GPR_EACH dw[k] = -__fdiv_rn(res[k], v[k]); }
+                        const bool w_too = !left || takes;
+                        if (gx_in_range(v) && (!w_too || gx_in_range(res))) {
+                            GPR_EACH du[k] = gx_recip(v[k]);
+                            if (w_too) { GPR_EACH dw[k] = -gx_quotient(res[k], v[k], du[k]); }
+                        } else {
+                            general_slopes<K>(res, v, du, dw, w_too);
+                        }
                         if (left) {
                             GPR_EACH { av[k] = adj_mul(adj[k], dw[k]); adj[k] = adj_mul(adj[k], du[k]); }
                         } else {
