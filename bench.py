@@ -908,7 +908,8 @@ def run_gpu(args, w):
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": kernel_ms / args.steps,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "f32",
         "data": "synthetic (seeded)",
-        "point_evals_per_s": value * w["nd"],
+        # points evaluated: a proposal whose values are the current state's takes its likelihood over
+        "point_evals_per_s": world * st["eval_points"] / (kernel_ms / 1e3),
         "config": config_of(args, w),
         "parallelism": "one population over %d GPUs (resampling cutoff exchanged per block, outside the "
                        "timed region)" % world if world > 1 else "1 GPU",

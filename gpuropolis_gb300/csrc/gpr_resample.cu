@@ -12,8 +12,8 @@
  *
  * This is integer and byte work over N doubles (1 MB at 131,072 chains): one
  * cluster of CTAs per segment holds the order-preserving 64-bit keys in
- * registers and radix-selects over them (8 bits per round), and one thread
- * per chain below the cutoff re-draws it.
+ * registers and radix-selects over them (8 bits per round), and a CTA re-draws
+ * a group of the chains below the cutoff in phases.
  */
 #include <cooperative_groups.h>
 #include <algorithm>
