@@ -32,6 +32,11 @@
 
 #define GPR_VERSION_STRING "gpuropolis-gb300 0.1 (sm_103a)"
 
+/* What the Hamiltonian kernel's layout was configured with (configure_hmc). */
+struct HmcLayout {
+    int wpc = 4, ctas_per_sm = 0, stream_mode = -1, G = 0;
+};
+
 struct gpr_handle {
     gpr_config cfg;
     int N = 0;
@@ -52,7 +57,7 @@ struct gpr_handle {
     /* selection scratch, allocated by the first gpr_resample/gpr_top_chains/gpr_map_chain */
     float* dscale = nullptr;               /* per-chain proposal scales          */
     float* dpart = nullptr;                /* chunk sums of the pipelined kernel for large datasets */
-    double* dgrad = nullptr;               /* results of gpr_loglik_grad (N * PL + N), kept when small */
+    double* dgrad = nullptr;               /* results and scratch of gpr_loglik_grad, kept when small */
     size_t dpart_floats = 0;
     double* dds_ns64 = nullptr;            /* batched data: unscaled normalising sums */
     int stream_data = 0;                   /* 1: always stream the dataset       */
@@ -81,6 +86,7 @@ struct gpr_handle {
 
     gpr::KParams kp;
     gpr::LaunchCfg lc;
+    HmcLayout hmc;
     int64_t launches = 0;
     std::string err;
 };
@@ -387,30 +393,34 @@ static int batched_wpc(const gpr::KParams& kp, int wpc, int pipe = 0) {
     return wpc;
 }
 
-/* The MH kernel with Hamiltonian constant moves: one chain per warp,
- * wpc0 warps per CTA, four points per lane per pass, a persistent grid of at
- * most ctas_per_sm CTAs per SM (0: as many as fit).  Capping the CTAs also
- * caps the shared-memory carveout, which leaves the rest of the SM's L1 to
- * the thread-local gradient tapes. */
-static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int stream_mode = -1) {
+/* The MH kernel with Hamiltonian constant moves: one chain per warp, wpc0 warps
+ * per CTA, 4 G points per lane and sweep (G 0: by hmc_passes), a persistent grid
+ * of at most ctas_per_sm CTAs per SM (0: as many as fit); capping them also caps
+ * the shared-memory carveout, which leaves the rest of the SM's L1 to what is
+ * spilled.
+ *
+ * stream_mode -1: the data are staged up to two passes and read from device
+ * memory beyond.  Staged / streamed, 65,536 chains: 128 points 0.92-0.98 (fixed
+ * programs and random ones of one variable; 1.06 random ones of three), 300
+ * points 0.96-1.18, 1,024 points 0.98-1.34, 2,048 points 1.10-1.48.  Streamed as
+ * well when asked, for batched data (each warp reads its own chain's dataset)
+ * and where staging does not fit. */
+#define GPR_HMC_STAGED_POINTS (2 * GPR_CHUNK_POINTS)
+
+static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int stream_mode = -1, int G = 0) {
     if (wpc0 < 1 || wpc0 > 8) wpc0 = 4;
     drop_graph(h);
     gpr::KParams& kp = h->kp;
     if (!gpr::grad_supported(kp))
         return fail(h, GPR_ERR_ARG, "gradient moves support program_length <= 127 (got %d)", kp.PL);
+    const int g = G > 0 ? G : gpr::hmc_passes(kp, h->num_sms);
     gpr::LaunchCfg lc;
-    lc.K = 4; lc.onepass = 0; lc.rolled = 0; lc.lockstep = 0; lc.carveout = 0; lc.pipe = 0;
-    /* Streamed when asked, for batched data (each warp reads its own chain's
-     * dataset from device memory), when staging does not fit, and when the
-     * staged copy would take over a quarter of the CTA's shared memory: the
-     * memory it frees goes to L1, which holds the gradient tapes (on the
-     * 1024-point rational model streaming measured 23% faster). */
-    const size_t staged = gpr::grad_smem_bytes(kp, wpc0, 0), streamed = gpr::grad_smem_bytes(kp, wpc0, 1);
-    lc.stream = h->stream_data || kp.nds > 0 || staged > 227 * 1024 ||
-                (stream_mode < 0 ? 4 * (staged - streamed) > staged : stream_mode > 0);
+    lc.K = 4 * g; lc.onepass = 0; lc.rolled = 0; lc.lockstep = 0; lc.carveout = 0; lc.pipe = 0;
+    lc.stream = h->stream_data || kp.nds > 0 || gpr::grad_smem_bytes(kp, g, wpc0, 0) > 227 * 1024 ||
+                (stream_mode < 0 ? kp.nd > GPR_HMC_STAGED_POINTS : stream_mode > 0);
     int wpc = wpc0;
-    size_t smem = gpr::grad_smem_bytes(kp, wpc, lc.stream);
-    while (smem > 227 * 1024 && wpc > 1) smem = gpr::grad_smem_bytes(kp, wpc /= 2, lc.stream);
+    size_t smem = gpr::grad_smem_bytes(kp, g, wpc, lc.stream);
+    while (smem > 227 * 1024 && wpc > 1) smem = gpr::grad_smem_bytes(kp, g, wpc /= 2, lc.stream);
     if (smem > 227 * 1024)
         return fail(h, GPR_ERR_ARG, "programs of length %d do not fit in shared memory", kp.PL);
     if (ctas_per_sm > 0) {
@@ -420,7 +430,7 @@ static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int s
         lc.carveout = (int)std::min(100.0, std::ceil(100.0 * need / (double)sm_smem));
     }
     int per_sm = 0;
-    CUDA_TRY(h, gpr::hmc_occupancy(kp, wpc, smem, lc.carveout, lc.stream, &per_sm));
+    CUDA_TRY(h, gpr::hmc_occupancy(kp, g, wpc, smem, lc.carveout, lc.stream, &per_sm));
     if (per_sm < 1) return fail(h, GPR_ERR_ARG, "kernel cannot be resident (smem %zu)", smem);
     if (ctas_per_sm > 0 && per_sm > ctas_per_sm) per_sm = ctas_per_sm;
     long long ctas = (long long)h->num_sms * per_sm;
@@ -430,6 +440,7 @@ static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int s
     lc.smem_bytes = smem;
     lc.ctas = (int)ctas;
     h->lc = lc;
+    h->hmc = {wpc0, ctas_per_sm, stream_mode, G};
     return GPR_OK;
 }
 
@@ -1043,6 +1054,8 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
     const gpr::LaunchCfg orig = h->lc;
     float best = 1e30f;
     gpr::LaunchCfg bestlc = orig;
+    const HmcLayout orig_hmc = h->hmc;
+    HmcLayout best_hmc = orig_hmc;
     cudaError_t e;
     /* trial blocks leave the per-chain scales alone */
     const float saved_target = h->kp.adapt_target;
@@ -1060,15 +1073,15 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
     AT_TRY(cudaMemcpyAsync(sSt, h->dstats, GPR_NSTATS * sizeof(unsigned long long), cudaMemcpyDeviceToDevice, h->stream));
     AT_TRY(cudaEventCreate(&e0));
     AT_TRY(cudaEventCreate(&e1));
-    /* the Hamiltonian kernel: CTA size and resident CTAs per SM, i.e. occupancy
-     * against L1 left for the gradient tapes */
+    /* the Hamiltonian kernel: passes per sweep, CTA size and resident CTAs per SM
+     * (occupancy against L1), each with the data staged (unless the handle
+     * always streams) and streamed */
     if (hmc) {
-        /* CTA size and residency cap, each with the data staged (unless the
-         * handle always streams) and streamed */
-        const int shapes[8][2] = {{4, 0}, {4, 7}, {4, 5}, {4, 4}, {2, 0}, {1, 0}, {8, 0}, {8, 3}};
+        const int shapes[8][3] = {{1, 4, 0}, {1, 1, 0}, {1, 8, 0}, {1, 4, 5}, {2, 4, 0}, {2, 1, 0}, {2, 8, 0}, {2, 4, 3}};
         for (int i = 0; i < 16; ++i) {
+            const int* sh = shapes[i % 8];
             const int want_stream = i >= 8;
-            if (configure_hmc(h, shapes[i % 8][0], shapes[i % 8][1], want_stream) != GPR_OK) continue;
+            if (configure_hmc(h, sh[1], sh[2], want_stream, sh[0]) != GPR_OK) continue;
             if (h->lc.stream != want_stream) continue;   /* forced one way: tried once */
             for (int rep = 0; rep < 2; ++rep) {
                 AT_TRY(cudaMemcpyAsync(h->dP, sP, cnt * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->stream));
@@ -1080,7 +1093,7 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
             }
             float ms = 0.0f;
             AT_TRY(cudaEventElapsedTime(&ms, e0, e1));
-            if (ms < best) { best = ms; bestlc = h->lc; }
+            if (ms < best) { best = ms; bestlc = h->lc; best_hmc = h->hmc; }
         }
         nc = 0;
     }
@@ -1136,6 +1149,7 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
         if (rc != GPR_OK) goto done;
     } else {
         h->lc = bestlc;
+        h->hmc = best_hmc;
     }
     AT_TRY(cudaMemcpyAsync(h->dP, sP, cnt * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->stream));
     AT_TRY(cudaMemcpyAsync(h->dC, sC, cnt * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
@@ -1150,7 +1164,7 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
 #undef AT_TRY
 done:
     h->kp.adapt_target = saved_target;
-    if (rc != GPR_OK) h->lc = orig;
+    if (rc != GPR_OK) { h->lc = orig; h->hmc = orig_hmc; }
     cudaFree(sP); cudaFree(sC); cudaFree(sPr); cudaFree(sLi); cudaFree(sSt);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -1243,6 +1257,12 @@ int gpr_set_moves(gpr_handle* h, int struct_every, float hmc_eps, int hmc_steps)
     h->kp.struct_every = struct_every;
     h->kp.hmc_eps = hmc_eps;
     h->kp.hmc_L = hmc_steps;
+    /* whether the programs are fixed decides the Hamiltonian kernel's width */
+    if (h->kp.const_mode == GPR_CONST_HMC && h->nd >= 0 && h->hmc.G == 0 &&
+        h->lc.K != 4 * gpr::hmc_passes(h->kp, h->num_sms)) {
+        CUDA_TRY(h, cudaSetDevice(h->device));
+        return configure_hmc(h, h->hmc.wpc, h->hmc.ctas_per_sm, h->hmc.stream_mode);
+    }
     return GPR_OK;
 }
 
@@ -1316,16 +1336,15 @@ int gpr_loglik_grad(gpr_handle* h, double* grad, double* likelihood) {
         return fail(h, GPR_ERR_ARG, "gradients support program_length <= 127 (got %d)", h->PL);
 
     CUDA_TRY(h, cudaSetDevice(h->device));
-    const size_t cnt = (size_t)h->N * h->PL, total = cnt + (size_t)h->N;
+    const size_t n = (size_t)h->N, cnt = n * h->PL;
+    const size_t total = cnt + n + (n + 2) / 2;   /* gradients, likelihoods, the launches' list of chains */
     const bool keep = total * sizeof(double) <= GPR_GRAD_KEEP_BYTES;
     double* buf = keep ? h->dgrad : nullptr;
     cudaError_t e = buf ? cudaSuccess : cudaMalloc(&buf, total * sizeof(double));
     if (keep && e == cudaSuccess) h->dgrad = buf;
     double* dg = buf;
     double* dl = e == cudaSuccess ? buf + cnt : nullptr;
-    /* batched data: every warp reads its chain's dataset from device memory */
-    const bool st = h->stream_data || h->kp.nds > 0 || gpr::grad_smem_bytes(h->kp, 4) > 227 * 1024;
-    if (e == cudaSuccess) e = gpr::launch_loglik_grad(h->kp, dg, dl, st, h->stream);
+    if (e == cudaSuccess) e = gpr::launch_loglik_grad(h->kp, h->num_sms, dg, dl, (int*)(dl + n), h->stream);
     if (e == cudaSuccess) {
         h->launches++;
         e = cudaMemcpyAsync(grad, dg, cnt * sizeof(double), cudaMemcpyDeviceToHost, h->stream);

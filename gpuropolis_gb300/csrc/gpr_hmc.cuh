@@ -34,22 +34,13 @@
 
 namespace gpr {
 
-/* Passes of 128 points (four per lane) that one sweep takes together: the
- * instructions are decoded once for G of them.  On the rational model (1,024
- * points) and on 16,384 points of three variables, with registers for 16 warps
- * per SM: 86 and 90 ms with 2, 94 and 100 ms with 1, 141 and 95 ms with 4; with
- * registers for 24 warps 115 and 105 ms with 2, 89 and 107 ms with 1. */
-#ifndef GPR_GRAD_G
-#define GPR_GRAD_G 2
-#endif
-/* Tape rows in shared memory (of G * 512 bytes per warp). */
-#ifndef GPR_GRAD_ROWS
-#define GPR_GRAD_ROWS 4
-#endif
-/* Resident CTAs of 8 warps per SM that the registers are allocated for. */
-#ifndef GPR_HMC_MIN_CTAS
-#define GPR_HMC_MIN_CTAS 2
-#endif
+/* The kernels come in two widths G: the passes of 128 points (four per lane)
+ * that one sweep takes together, its instructions decoded once for all of them.
+ * G = 2 has registers for 16 warps per SM and leaves an odd last pass to the
+ * sweep of one; G = 1 has registers for 32.  Which is used: hmc_passes and
+ * launch_loglik_grad (gpr_hmc.cu).  Results do not depend on it. */
+__host__ __device__ constexpr int hmc_min_ctas(int G) { return G == 1 ? 4 : 2; }   /* of 8 warps, per SM */
+#define GPR_GRAD_ROWS 4      /* tape rows in shared memory, of G * 512 bytes per warp */
 #define GPR_GRAD_CONSTS 8    /* constants whose shares are reduced together */
 #define GPR_GRAD_STRIDE 36   /* floats between their rows of lane shares: conflict-free reads of the reduction */
 
@@ -72,6 +63,8 @@ namespace gpr {
 #define GW_X3 252u
 #define GW_NODE_ONE 254u
 #define GW_NODE_NAN 255u
+#define GW_CONSTS 0xffff     /* of grad_prepare's result: the constants the program reads */
+#define GW_LONG 0x10000      /* ... whether it has a power, exp, log, root or trigonometric op */
 
 /* Per-warp shared memory of the gradient evaluator and the HMC kernel. */
 struct GradSmem {
@@ -93,94 +86,135 @@ struct GradSmem {
 
 __host__ __device__ __forceinline__ size_t grad_rows_bytes(int PL) { return align16((size_t)PL * 4); }
 
-__host__ __device__ __forceinline__ size_t grad_warp_bytes(int PL, int max_instr) {
-    const size_t plp = align16((size_t)PL);
+/* G passes at a time; block: with the buffers that only the MH block has (the
+ * proposal's ops, constants and program, the current gradient, the momentum). */
+__host__ __device__ __forceinline__ size_t grad_warp_bytes(int PL, int max_instr, int G, bool block) {
+    const size_t plp = align16((size_t)PL), n = block ? 2 : 1;
     size_t b = 0;
-    b += 2 * plp;                                              /* ops */
-    b += align16(2 * plp * 4);                                 /* Cs */
-    b += align16(2 * (size_t)max_instr * sizeof(gpr_word));    /* prog */
+    b += n * plp;                                              /* ops */
+    b += align16(n * plp * 4);                                 /* Cs */
+    b += align16(n * (size_t)max_instr * sizeof(gpr_word));    /* prog */
     b += align16((size_t)max_instr * 4);                       /* gprog */
     b += align16((size_t)max_instr * 8);                       /* eprog */
     b += 16;                                                   /* cnode */
     b += grad_rows_bytes(PL);                                  /* gradient sums */
-    b += 3 * align16(plp * 4);                                 /* gcur, gnew, mom */
-    b += (size_t)GPR_GRAD_ROWS * GPR_GRAD_G * 512;             /* rows */
-    b += (size_t)GPR_GRAD_G * GPR_GRAD_CONSTS * GPR_GRAD_STRIDE * 4;   /* share */
+    b += (block ? 3 : 1) * align16(plp * 4);                   /* gnew, gcur, mom */
+    b += (size_t)GPR_GRAD_ROWS * G * 512;                      /* rows */
+    b += (size_t)G * GPR_GRAD_CONSTS * GPR_GRAD_STRIDE * 4;    /* share */
     return align16(b);
 }
 
-__device__ __forceinline__ GradSmem carve_grad(uint8_t* base, int PL, int max_instr) {
+__device__ __forceinline__ GradSmem carve_grad(uint8_t* base, int PL, int max_instr, int G, bool block) {
     GradSmem w;
-    const size_t plp = align16((size_t)PL);
+    const size_t plp = align16((size_t)PL), n = block ? 2 : 1;
     uint8_t* p = base;
-    w.ops[0] = p; w.ops[1] = p + plp; p += 2 * plp;
-    w.Cs[0] = (float*)p; w.Cs[1] = (float*)p + plp; p += align16(2 * plp * 4);
-    w.prog[0] = (gpr_word*)p; w.prog[1] = (gpr_word*)p + max_instr; p += align16(2 * (size_t)max_instr * sizeof(gpr_word));
+    w.ops[0] = p; w.ops[1] = block ? p + plp : nullptr; p += n * plp;
+    w.Cs[0] = (float*)p; w.Cs[1] = block ? (float*)p + plp : nullptr; p += align16(n * plp * 4);
+    w.prog[0] = (gpr_word*)p; w.prog[1] = block ? (gpr_word*)p + max_instr : nullptr;
+    p += align16(n * (size_t)max_instr * sizeof(gpr_word));
     w.gprog = (uint32_t*)p; p += align16((size_t)max_instr * 4);
     w.eprog = (uint2*)p; p += align16((size_t)max_instr * 8);
     w.cnode = p; p += 16;
     w.gacc = (float*)p; p += grad_rows_bytes(PL);
-    w.gcur = (float*)p; p += align16(plp * 4);
     w.gnew = (float*)p; p += align16(plp * 4);
-    w.mom = (float*)p; p += align16(plp * 4);
-    w.rows = (float*)p; p += (size_t)GPR_GRAD_ROWS * GPR_GRAD_G * 512;
+    w.gcur = w.mom = nullptr;
+    if (block) {
+        w.gcur = (float*)p; p += align16(plp * 4);
+        w.mom = (float*)p; p += align16(plp * 4);
+    }
+    w.rows = (float*)p; p += (size_t)GPR_GRAD_ROWS * G * 512;
     w.share = (float*)p;
     return w;
 }
 
+/* An instruction of the adjoint before it has its rows.  A result is kept only
+ * if the way back reads it: the factor of a product whose other factor is a
+ * constant or popped, an argument or a result where a derivative is written in
+ * it, and every pushed value. */
+struct GradWord {
+    uint32_t code, node;
+    bool arg, res;      /* the accumulator before, after is read on the way back */
+    bool share;         /* it reads a constant that the program owns              */
+};
+__device__ __forceinline__ GradWord grad_word(uint32_t ins) {
+    GradWord g;
+    g.code = ins & 0xffu;
+    g.node = (ins >> 8) & 0xffu;
+    g.arg = g.res = false;
+    if (g.code == I_LD1 || g.code == I_LDNAN) {
+        g.node = g.code == I_LD1 ? GW_NODE_ONE : GW_NODE_NAN;
+        g.code = I_LDC;
+    }
+    g.share = g.code == I_LDC && g.node < GW_NODE_ONE;
+    if (GPR_IS_BIN(g.code)) {
+        const uint32_t bop = GPR_BIN_BOP(g.code), left = GPR_BIN_ACCLEFT(g.code);
+        uint32_t src = GPR_CODE_SRC(g.code);
+        if (src == SRC_ONE) { src = SRC_C; g.node = GW_NODE_ONE; }
+        g.code = GW_CODE(bop, left, src);
+        g.share = src == SRC_C && g.node < GW_NODE_ONE;
+        const bool takes = src == SRC_POP || g.share;      /* the operand has a share */
+        if (bop == BOP_MUL) g.arg = takes;
+        else if (bop == BOP_DIV) { g.arg = !left; g.res = !left || takes; }
+        else if (bop == BOP_POW) { g.arg = left || takes; g.res = !left || takes; }
+    } else if (g.code == I_PUSH) {
+        g.res = true;
+    } else if (g.code >= U_INV) {
+        g.res = g.code == U_INV || g.code == U_EXP || g.code == U_SQRT || g.code == U_TAN;
+        g.arg = !g.res;
+    }
+    return g;
+}
+
 /* The adjoint words of a compiled program, into ws.gprog; returns how many
- * constants it reads.  A result is kept only if the way back reads it: the
- * factor of a product whose other factor is a constant or popped, an argument
- * or a result where a derivative is written in it, and every pushed value. */
-static __device__ int grad_prepare(const gpr_word* prog, int ninstr, const GradSmem& ws, int lane) {
-    int nconst = 0;
-    if (lane == 0) {
-        uint8_t st[32];      /* instructions of the pushes pending: at most floor(log2(PL / 2)) + 1 */
-        int sp = 0, rows = 0;
-        uint32_t before = 0u;    /* the word of instruction i - 1, not stored yet */
+ * constants it reads (GW_CONSTS) and whether it has a long op (GW_LONG).  A lane
+ * per instruction: rows and constants are numbered by ballots, and only the
+ * pushes and pops are paired one after the other.  As one lane's walk, after
+ * every change of structure, it held a warp up for a tenth of a move: 65,536
+ * chains of random programs on 30 points, 8 leapfrog steps: 55.1 -> 51.0 ms. */
+static __device__ __noinline__ int grad_prepare(const gpr_word* prog, int ninstr, const GradSmem& ws, int lane) {
+    const uint32_t below = (1u << lane) - 1u;
+    int nconst = 0, rows = 0, sp = 0;
+    bool heavy = false;
+    uint32_t pending = 0u;       /* lane d: the row of the push pending at depth d (fewer than 32) */
 #pragma unroll 1
-        for (int i = 0; i < ninstr; ++i) {
-            uint32_t code = prog[i] & 0xffu, node = (prog[i] >> 8) & 0xffu;
-            uint32_t aux = GW_NONE, row = GW_NONE;
-            bool need_arg = false, need_res = false;   /* the accumulator before, after */
-            if (code == I_LD1 || code == I_LDNAN) {
-                node = code == I_LD1 ? GW_NODE_ONE : GW_NODE_NAN;
-                code = I_LDC;
-            }
-            bool takes = code == I_LDC;                 /* a constant or a popped value has a share */
-            if (GPR_IS_BIN(code)) {
-                const uint32_t bop = GPR_BIN_BOP(code), left = GPR_BIN_ACCLEFT(code);
-                uint32_t src = GPR_CODE_SRC(code);
-                if (src == SRC_ONE) { src = SRC_C; node = GW_NODE_ONE; }
-                code = GW_CODE(bop, left, src);
-                takes = src == SRC_POP || (src == SRC_C && node < GW_NODE_ONE);
-                if (src == SRC_POP) { --sp; aux = GW_ROW(ws.gprog[st[sp]]); }
-                if (bop == BOP_MUL) need_arg = takes;
-                else if (bop == BOP_DIV) { need_arg = !left; need_res = !left || takes; }
-                else if (bop == BOP_POW) { need_arg = left || takes; need_res = !left || takes; }
-                if (src != SRC_C) takes = false;
-            } else if (code == I_PUSH) {
-                need_res = true;
-            } else if (code >= U_INV) {
-                need_res = code == U_INV || code == U_EXP || code == U_SQRT || code == U_TAN;
-                need_arg = !need_res;
-            } else if (code == I_LDX || code == I_LDX2 || code == I_LDX3) {
-                row = code == I_LDX ? GW_X1 : code == I_LDX2 ? GW_X2 : GW_X3;
-            }
-            if (takes && node < GW_NODE_ONE) {
-                if (nconst < GPR_GRAD_CONSTS) ws.cnode[nconst] = (uint8_t)node;
-                aux = (uint32_t)nconst++;
-            }
-            if (need_arg && GW_ROW(before) == GW_NONE) before = (before & 0xff00ffffu) | ((uint32_t)rows++ << 16);
-            if (i > 0) ws.gprog[i - 1] = before;
-            if (need_res) row = (uint32_t)rows++;
-            if (code == I_PUSH) { ws.gprog[i] = row << 16; st[sp++] = (uint8_t)i; }
-            before = code | (node << 8) | (row << 16) | (aux << 24);
+    for (int base = 0; base < ninstr; base += 32) {
+        const int i = base + lane;
+        const bool in = i < ninstr;
+        /* the last instruction is I_END, which keeps and reads nothing */
+        const GradWord g = grad_word(in ? prog[i] : (uint32_t)I_END);
+        bool next_arg = __shfl_down_sync(FULLMASK, (int)g.arg, 1) != 0;
+        if (lane == 31) next_arg = i + 1 < ninstr && grad_word(prog[i + 1]).arg;
+        uint32_t row = g.code == I_LDX ? GW_X1 : g.code == I_LDX2 ? GW_X2 : g.code == I_LDX3 ? GW_X3 : GW_NONE;
+        const bool keep = g.res || (next_arg && row == GW_NONE);
+        const uint32_t kept = __ballot_sync(FULLMASK, keep), shares = __ballot_sync(FULLMASK, g.share);
+        if (keep) row = (uint32_t)(rows + __popc(kept & below));
+        rows += __popc(kept);
+        uint32_t aux = GW_NONE;
+        if (g.share) {
+            aux = (uint32_t)(nconst + __popc(shares & below));
+            if (aux < GPR_GRAD_CONSTS) ws.cnode[aux] = (uint8_t)g.node;
         }
-        ws.gprog[ninstr - 1] = before;
+        nconst += __popc(shares);
+        heavy = heavy || (g.code >= GW_BIN ? GW_BOP(g.code) == BOP_POW : g.code > U_INV && g.code < U_ABS);
+        const uint32_t push = __ballot_sync(FULLMASK, g.code == I_PUSH);
+        uint32_t todo = push | __ballot_sync(FULLMASK, g.code >= GW_BIN && GW_SRC(g.code) == SRC_POP);
+#pragma unroll 1
+        for (; todo; todo &= todo - 1u) {
+            const int b = __ffs(todo) - 1;
+            if ((push >> b) & 1u) {
+                const uint32_t r = __shfl_sync(FULLMASK, row, b);
+                if (lane == sp) pending = r;
+                ++sp;
+            } else {
+                --sp;
+                const uint32_t r = __shfl_sync(FULLMASK, pending, sp);
+                if (lane == b) aux = r;
+            }
+        }
+        if (in) ws.gprog[i] = g.code | (g.node << 8) | (row << 16) | (aux << 24);
     }
     __syncwarp();
-    return __shfl_sync(FULLMASK, nconst, 0);
+    return nconst | (__any_sync(FULLMASK, heavy) ? GW_LONG : 0);
 }
 
 /* The words paired with the constants at hand. */
@@ -573,42 +607,24 @@ __device__ __forceinline__ float reduce_shares(const float* share, int g, int la
     return __fadd_rn(v, __shfl_xor_sync(FULLMASK, v, 1));
 }
 
-/* Log-likelihood of one program (double-float at scale 2^-64, -inf when any
- * point is invalid, as eval_loglik) and its gradient over all PL constants:
- * g[i] = 2^-64 d loglik / d C[i] in FP32, at the bookkeeping scale like the
- * likelihood (0 for constants the program does not read).  The gradient is
- * meaningful only when the likelihood is finite.  nconst: constants the
- * program reads (grad_prepare).
- *
- * Bound by issued instructions, most of them the interpreter's, and by their
- * latency: hence only the rows that are read again are kept, and in shared
- * memory (a row for every instruction in thread-local memory made 8 GB of
- * DRAM writes per 44 ms), an instruction is decoded once for G passes, sums
- * and products with a constant or x take their operand where it is, and the
- * constants' shares are reduced together.  65,536 chains of the rational model,
- * 1,024 points, 10 moves of 8 leapfrog steps: 146 -> 82 ms; their gradients
- * alone 1.86 -> 1.0 ms. */
-template <int MAXR, int NV, bool STREAM>
-static __device__ __noinline__ df eval_loglik_grad(const uint2* prog, int ninstr, int nconst, const GradSmem ws,
-                                                   const DataView dv, const KParams& p, int lane, int& pts_out,
-                                                   float* g) {
-    constexpr int G = GPR_GRAD_G, K = 4 * G;
-    const int PL = p.PL;
-    float4 local_rows[MAXR * G];   /* rows beyond the warp's: a program of PL nodes keeps at most 3 PL / 2 */
+/* What the sweeps of a program leave. */
+struct GradSums {
+    float s, mine;       /* this lane's share of S; lanes 4j..4j+3: the sum of constant j */
+    int pts;
+    bool bad;
+};
+
+/* Passes [pass, end) of a program, G at a time (a multiple of G of them). */
+template <int G, int NV, bool STREAM>
+__device__ __forceinline__ void grad_passes_of(const uint2* prog, int ninstr, int nconst, float4* local_rows,
+                                               const GradSmem& ws, const DataView& dv, float w_to_df, int lane,
+                                               int pass, int end, GradSums& sum) {
+    constexpr int K = 4 * G;
     Tape<K> tape;
     tape.sm = (float4*)ws.rows + lane;
     tape.local = local_rows;
 #pragma unroll 1
-    for (int j = lane; j < PL; j += 32) ws.gacc[j] = 0.0f;
-    __syncwarp();
-    const float w_to_df = p.w_to_df;
-    int pts = 0;
-    float s = 0.0f;
-    float mine = 0.0f;             /* lanes 4j..4j+3: the sum of constant j */
-    bool bad = false;
-    const int npass = (dv.nd + 127) / 128;
-#pragma unroll 1
-    for (int pass = 0; pass < npass && !bad; pass += G) {
+    for (; pass < end && !sum.bad; pass += G) {
         float x[NV][K], adj[K];
         load_points<K, NV, STREAM>(dv, pass, lane, x);
         forward_tape<K, NV>(prog, ninstr, x, tape, adj);
@@ -616,7 +632,7 @@ static __device__ __noinline__ df eval_loglik_grad(const uint2* prog, int ninstr
 #pragma unroll
         for (int gi = 0; gi < G; ++gi) {
             const int left = dv.nd - (pass + gi) * GPR_CHUNK_POINTS;
-            if (bad || left <= 0) {
+            if (sum.bad) {
 #pragma unroll
                 for (int k = 4 * gi; k < 4 * gi + 4; ++k) adj[k] = 0.0f;
                 continue;
@@ -630,7 +646,7 @@ static __device__ __noinline__ df eval_loglik_grad(const uint2* prog, int ninstr
                 const float r = __fsub_rn(adj[4 * gi + kk], y[kk]);
                 const float q = __fmul_rn(r, r);
                 b |= !(q <= FLT_MAX);
-                s = fmaf(q, wi, s);
+                sum.s = fmaf(q, wi, sum.s);
                 adj[4 * gi + kk] = __fmul_rn(__fmul_rn(-2.0f, wi), r);
             };
             if (left >= GPR_CHUNK_POINTS) {
@@ -643,9 +659,9 @@ static __device__ __noinline__ df eval_loglik_grad(const uint2* prog, int ninstr
                     else adj[4 * gi + kk] = 0.0f;
                 }
             }
-            pts += min(GPR_CHUNK_POINTS, left);
-            bad = __any_sync(FULLMASK, b);
-            if (bad) {
+            sum.pts += min(GPR_CHUNK_POINTS, left);
+            sum.bad = __any_sync(FULLMASK, b);
+            if (sum.bad) {
 #pragma unroll
                 for (int k = 4 * gi; k < 4 * gi + 4; ++k) adj[k] = 0.0f;
             } else {
@@ -657,20 +673,52 @@ static __device__ __noinline__ df eval_loglik_grad(const uint2* prog, int ninstr
             if (nconst > 0) {
                 __syncwarp();
 #pragma unroll
-                for (int gi = 0; gi < G; ++gi) mine = __fadd_rn(mine, reduce_shares(ws.share, gi, lane));
+                for (int gi = 0; gi < G; ++gi) sum.mine = __fadd_rn(sum.mine, reduce_shares(ws.share, gi, lane));
                 __syncwarp();
             }
         }
     }
+}
+
+/* Log-likelihood of one program (double-float at scale 2^-64, -inf when any
+ * point is invalid, as eval_loglik) and its gradient over all PL constants:
+ * g[i] = 2^-64 d loglik / d C[i] in FP32, at the bookkeeping scale like the
+ * likelihood (0 for constants the program does not read).  The gradient is
+ * meaningful only when the likelihood is finite.  info: of grad_prepare.
+ *
+ * Bound by issued instructions, most of them the interpreter's, and by their
+ * latency: hence only the rows that are read again are kept, and in shared
+ * memory (a row for every instruction in thread-local memory made 8 GB of
+ * DRAM writes per 44 ms), an instruction is decoded once for G passes, sums
+ * and products with a constant or x take their operand where it is, and the
+ * constants' shares are reduced together.  65,536 chains of the rational model,
+ * 1,024 points, 10 moves of 8 leapfrog steps: 146 -> 82 ms; their gradients
+ * alone 1.86 -> 1.0 ms. */
+template <int MAXR, int G, int NV, bool STREAM>
+__device__ __forceinline__ df eval_loglik_grad(const uint2* prog, int ninstr, int info, const GradSmem& ws,
+                                               const DataView& dv, const KParams& p, int lane, int& pts_out, float* g) {
+    const int PL = p.PL, nconst = info & GW_CONSTS;
+    float4 local_rows[MAXR * G];   /* rows beyond the warp's: a program of PL nodes keeps at most 3 PL / 2 */
+#pragma unroll 1
+    for (int j = lane; j < PL; j += 32) ws.gacc[j] = 0.0f;
+    __syncwarp();
+    GradSums sum = {0.0f, 0.0f, 0, false};
+    const int npass = (dv.nd + 127) / 128;
+    int pass = 0;
+    if constexpr (G > 1) {
+        pass = npass / G * G;
+        grad_passes_of<G, NV, STREAM>(prog, ninstr, nconst, local_rows, ws, dv, p.w_to_df, lane, 0, pass, sum);
+    }
+    grad_passes_of<1, NV, STREAM>(prog, ninstr, nconst, local_rows, ws, dv, p.w_to_df, lane, pass, npass, sum);
     __syncwarp();
 #pragma unroll 1
     for (int c = lane; c < PL; c += 32) g[c] = ws.gacc[c];
     __syncwarp();
-    if ((lane & 3) == 0 && (lane >> 2) < nconst) g[ws.cnode[lane >> 2]] = mine;
+    if ((lane & 3) == 0 && (lane >> 2) < nconst) g[ws.cnode[lane >> 2]] = sum.mine;
     __syncwarp();
-    pts_out = pts;
-    if (bad) return df_make(-INFINITY, 0.0f);
-    df S = warp_sum_df(df_make(s, 0.0f));
+    pts_out = sum.pts;
+    if (sum.bad) return df_make(-INFINITY, 0.0f);
+    df S = warp_sum_df(df_make(sum.s, 0.0f));
     if (!isfinite(S.hi)) return df_make(-INFINITY, 0.0f);
     return df_sub(df_neg(S), df_make(dv.ns_hi, dv.ns_lo));
 }
@@ -702,9 +750,6 @@ __device__ __forceinline__ void hmc_jitter_uniforms(uint32_t seed, uint32_t chai
     u2 = __fmul_rn((float)(c[1] >> 8), 5.9604644775390625e-08f);
 }
 
-/* ------------------------------------------------------------------------ */
-/* d loglik / d C for every chain's current state (gpr_loglik_grad): one warp
- * per chain, grad[i*N + chain] (double, unscaled) and lik[chain]. */
 /* The dataset: staged into this CTA's shared memory, or (STREAM) read from
  * device memory.  Returns where the per-warp regions start, or nullptr (the
  * same in every thread) when the staging copy timed out. */
@@ -717,19 +762,28 @@ __device__ __forceinline__ uint8_t* grad_dataset(uint8_t* smem, const KParams& p
     return smem + GPR_STAGED_OFFSET + align16((size_t)data_arrays(p) * p.nd_pad * 4);
 }
 
-template <int MAXR, bool STREAM, int NV>
-__global__ void __launch_bounds__(128, 2 * GPR_HMC_MIN_CTAS) loglik_grad_kernel(const __grid_constant__ KParams p, double* grad,
-                                                          double* lik_out) {
+/* ------------------------------------------------------------------------ */
+/* d loglik / d C for every chain's current state (gpr_loglik_grad): one warp
+ * per chain, grad[i*N + chain] (double, unscaled) and lik[chain].  A chain reads
+ * every point once, so the data are read from device memory.  later (may be
+ * null): a list of chains, its length first; the kernel with G = 2 leaves the
+ * programs with a long op there, the one with G = 1 takes the listed ones. */
+template <int MAXR, int G, int NV>
+__global__ void __launch_bounds__(128, 2 * hmc_min_ctas(G)) loglik_grad_kernel(const __grid_constant__ KParams p,
+                                                                              double* grad, double* lik_out,
+                                                                              int* later) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
-    DataView dv;
-    uint8_t* wbase = grad_dataset<STREAM>(smem, p, dv);
-    if (!wbase) return;   /* the staging copy timed out: the error flag is set */
-    const GradSmem ws = carve_grad(wbase + (size_t)warp * grad_warp_bytes(p.PL, p.max_instr), p.PL, p.max_instr);
-    const int chain = blockIdx.x * (blockDim.x >> 5) + warp;
+    int chain = blockIdx.x * (blockDim.x >> 5) + warp;
+    if (G == 1 && later) {
+        if (chain >= later[0]) return;
+        chain = later[1 + chain];
+    }
     if (chain >= p.N) return;
-    if (STREAM && p.nds > 0) dv = data_view(p, nullptr, true, chain_dataset(p, chain));   /* batched: streamed */
+    const GradSmem ws = carve_grad(smem + (size_t)warp * grad_warp_bytes(p.PL, p.max_instr, G, false), p.PL,
+                                   p.max_instr, G, false);
+    const DataView dv = data_view(p, nullptr, true, p.nds > 0 ? chain_dataset(p, chain) : -1);
     const int PL = p.PL;
     for (int i = lane; i < PL; i += 32) {
         const int o = p.P[(size_t)i * p.N + chain];
@@ -739,11 +793,15 @@ __global__ void __launch_bounds__(128, 2 * GPR_HMC_MIN_CTAS) loglik_grad_kernel(
     __syncwarp();
     const CompileOut co = compile_parallel<NV>(ws.ops[0], PL, ws.prog[0], compile_scratch(ws.rows, PL), lane);
     __syncwarp();
-    const int nconst = grad_prepare(ws.prog[0], co.ninstr, ws, lane);
+    const int info = grad_prepare(ws.prog[0], co.ninstr, ws, lane);
+    if (G > 1 && later && (info & GW_LONG)) {
+        if (lane == 0) later[1 + atomicAdd(later, 1)] = chain;
+        return;
+    }
     build_grad_program(ws.gprog, ws.Cs[0], co.ninstr, ws.eprog, lane);
     __syncwarp();
     int pts = 0;
-    const df lik = eval_loglik_grad<MAXR, NV, STREAM>(ws.eprog, co.ninstr, nconst, ws, dv, p, lane, pts, ws.gnew);
+    const df lik = eval_loglik_grad<MAXR, G, NV, true>(ws.eprog, co.ninstr, info, ws, dv, p, lane, pts, ws.gnew);
     for (int i = lane; i < PL; i += 32) grad[(size_t)i * p.N + chain] = (double)ws.gnew[i] * GPR_DF_UNSCALE;
     if (lane == 0) lik_out[chain] = df_to_double_unscaled(lik);
 }
@@ -757,19 +815,28 @@ static __device__ __noinline__ CompileOut compile_apart(const uint8_t* ops, int 
     return compile_parallel<NV>(ops, PL, prog, cs, lane);
 }
 
+/* The gradient out of line, called from two places.  (The gradient kernel,
+ * with one, has it inline: the call's arguments go through local memory.) */
+template <int MAXR, int G, int NV, bool STREAM>
+static __device__ __noinline__ df eval_apart(const uint2* prog, int ninstr, int info, const GradSmem ws,
+                                             const DataView dv, const KParams& p, int lane, int& pts, float* g) {
+    return eval_loglik_grad<MAXR, G, NV, STREAM>(prog, ninstr, info, ws, dv, p, lane, pts, g);
+}
+
 /* ------------------------------------------------------------------------ */
 /* The MH block with Hamiltonian constant moves.  One warp per chain, chains
- * claimed from the global counter; evaluation with the adjoint on K points
+ * claimed from the global counter; evaluation with the adjoint on 4 G points
  * per lane. */
-template <int MAXR, int RNG, bool STREAM, int NV>
-__global__ void __launch_bounds__(256, GPR_HMC_MIN_CTAS) mh_hmc_kernel(const __grid_constant__ KParams p) {
+template <int MAXR, int G, int RNG, bool STREAM, int NV>
+__global__ void __launch_bounds__(256, hmc_min_ctas(G)) mh_hmc_kernel(const __grid_constant__ KParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     DataView dv;
     uint8_t* wbase = grad_dataset<STREAM>(smem, p, dv);
     if (!wbase) return;   /* the staging copy timed out: the error flag is set */
-    const GradSmem ws = carve_grad(wbase + (size_t)warp * grad_warp_bytes(p.PL, p.max_instr), p.PL, p.max_instr);
+    const GradSmem ws = carve_grad(wbase + (size_t)warp * grad_warp_bytes(p.PL, p.max_instr, G, true), p.PL,
+                                   p.max_instr, G, true);
     const int PL = p.PL;
     const bool adapt = p.chain_scale && p.adapt_target > 0.0f;
     const uint32_t seed = p.seed;
@@ -841,7 +908,7 @@ __global__ void __launch_bounds__(256, GPR_HMC_MIN_CTAS) mh_hmc_kernel(const __g
                     prepared = gbuf;
                     build_grad_program(ws.gprog, ws.Cs[ccur], co.ninstr, ws.eprog, lane);
                     __syncwarp();
-                    lik = eval_loglik_grad<MAXR, NV, STREAM>(ws.eprog, co.ninstr, nconst, ws, dv, p, lane, pe, ws.gnew);
+                    lik = eval_apart<MAXR, G, NV, STREAM>(ws.eprog, co.ninstr, nconst, ws, dv, p, lane, pe, ws.gnew);
                 }
                 const df backward = df_make(__fmul_rn(-p.logcount[co.count], GPR_DF_SCALE), 0.0f);
                 st_pts += (unsigned)pe;
@@ -911,7 +978,7 @@ __global__ void __launch_bounds__(256, GPR_HMC_MIN_CTAS) mh_hmc_kernel(const __g
                         build_grad_program(ws.gprog, q, cur_ninstr, ws.eprog, lane);
                         __syncwarp();
                         int pe = 0;
-                        lik = eval_loglik_grad<MAXR, NV, STREAM>(ws.eprog, cur_ninstr, nconst, ws, dv, p, lane, pe, ws.gnew);
+                        lik = eval_apart<MAXR, G, NV, STREAM>(ws.eprog, cur_ninstr, nconst, ws, dv, p, lane, pe, ws.gnew);
                         st_pts += (unsigned)pe;
                         st_evals++; st_nodes += (unsigned)cur_count;
                         st_np += (unsigned long long)(cur_count + 4) * (unsigned)pe;
@@ -986,8 +1053,8 @@ __global__ void __launch_bounds__(256, GPR_HMC_MIN_CTAS) mh_hmc_kernel(const __g
 }
 
 /* The kernels for three input variables (gpr_hmc_v.cu). */
-const void* grad_kernel_v3(int maxr, int stream);
-const void* hmc_kernel_v3(const KParams& p, int stream);
+const void* grad_kernel_v3(int maxr, int G);
+const void* hmc_kernel_v3(const KParams& p, int G, int stream);
 
 }  // namespace gpr
 

@@ -187,12 +187,15 @@ cudaError_t launch_math(int op, const float* a, const float* b, float* out, int 
 cudaError_t time_fp_adds(int iters, float* ms_d32, float* ms_d1, float* ms_f32);
 
 /* Gradient of the log-likelihood and the MH kernel with Hamiltonian constant
- * moves (gpr_hmc.cu).  grad_smem_bytes: dynamic shared memory of either for
- * a CTA of warps_per_cta chains. */
-size_t grad_smem_bytes(const KParams& p, int warps_per_cta, int stream = 0);
+ * moves (gpr_hmc.cu), on a device of sms SMs.  hmc_passes: the passes that a
+ * sweep of the Hamiltonian kernel takes together (G, 1 or 2); grad_smem_bytes:
+ * its dynamic shared memory for a CTA of warps_per_cta chains.  later: N + 1
+ * ints of scratch. */
+int hmc_passes(const KParams& p, int sms);
+size_t grad_smem_bytes(const KParams& p, int G, int warps_per_cta, int stream);
 bool grad_supported(const KParams& p);   /* PROGRAM_LENGTH <= 127 */
-cudaError_t launch_loglik_grad(const KParams& p, double* grad, double* lik, int stream, cudaStream_t st);
-cudaError_t hmc_occupancy(const KParams& p, int warps_per_cta, size_t smem, int carveout, int stream,
+cudaError_t launch_loglik_grad(const KParams& p, int sms, double* grad, double* lik, int* later, cudaStream_t st);
+cudaError_t hmc_occupancy(const KParams& p, int G, int warps_per_cta, size_t smem, int carveout, int stream,
                           int* ctas_per_sm);
 cudaError_t launch_hmc_block(const KParams& p, const LaunchCfg& lc, cudaStream_t st);
 
