@@ -444,6 +444,22 @@ static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int s
     return GPR_OK;
 }
 
+/* A layout in force: the launch configuration and the kernel parameters that
+ * only fit it.  The rows at h->dpart serve every layout configured so far. */
+struct Layout {
+    gpr::LaunchCfg lc;
+    HmcLayout hmc;
+    int part_stride, ppt;
+};
+static Layout layout_of(const gpr_handle* h) { return {h->lc, h->hmc, h->kp.part_stride, h->kp.ppt}; }
+static void commit_layout(gpr_handle* h, const Layout& l) {
+    h->lc = l.lc;
+    h->hmc = l.hmc;
+    h->kp.part = h->dpart;
+    h->kp.part_stride = l.part_stride;
+    h->kp.ppt = l.ppt;
+}
+
 /* A dataset is streamed from device memory when the caller asks for it (or
  * choose_launch does), or when staging it beside a full CTA of warps would not fit in shared memory;
  * streaming uses K = 4 points per lane in passes.  pipe: the pipelined kernel
@@ -500,25 +516,21 @@ static int configure_launch(gpr_handle* h, int K, int onepass, int rolled, int l
     lc.ctas = (int)ctas;
     /* chunk sums beyond the kernel's shared-memory board: one row per chain in
      * flight (8 per CTA, 16 of the pipelined kernel) in device memory */
-    kp.part_stride = 0;
     const bool many = !pipe && lc.K == 8 && lc.stream;
-    const int passes = (kp.nd + 32 * lc.K - 1) / (32 * lc.K);
-    kp.ppt = std::max(1, (passes + GPR_TASKS - 1) / GPR_TASKS);
     const int stride = pipe ? gpr::pipe_part_stride(kp.nd) : many ? gpr::mh_part_stride(kp.nd) : 0;
-    if (stride > 0) {
-        const size_t need_f = (size_t)lc.ctas * (pipe ? 16 : 8) * (size_t)stride;
-        if (h->dpart_floats < need_f) {
-            CUDA_TRY(h, cudaStreamSynchronize(h->stream));
-            cudaFree(h->dpart);
-            h->dpart = nullptr;
-            h->dpart_floats = 0;
-            CUDA_TRY(h, cudaMalloc(&h->dpart, need_f * sizeof(float)));
-            h->dpart_floats = need_f;
-        }
-        kp.part = h->dpart;
-        kp.part_stride = stride;
+    const size_t need_f = (size_t)lc.ctas * (pipe ? 16 : 8) * (size_t)stride;
+    if (h->dpart_floats < need_f) {
+        float* part = nullptr;
+        CUDA_TRY(h, cudaMalloc(&part, need_f * sizeof(float)));
+        cudaStreamSynchronize(h->stream);      /* a block may be using the old rows */
+        cudaFree(h->dpart);
+        h->dpart = part;
+        h->dpart_floats = need_f;
     }
-    h->lc = lc;
+    /* nothing can fail any more: the layout and the parameters that go with it
+     * change together, so a failed call leaves those of the layout in force */
+    const int passes = (kp.nd + 32 * lc.K - 1) / (32 * lc.K);
+    commit_layout(h, {lc, h->hmc, stride, std::max(1, (passes + GPR_TASKS - 1) / GPR_TASKS)});
     return GPR_OK;
 }
 
@@ -571,6 +583,14 @@ static int choose_launch(gpr_handle* h) {
     rc = configure_streamed(h, 4, pipe);
     if (rc == GPR_OK && h->lc.ctas > staged) return rc;
     return configure_launch(h, 4, 0, 0, 1, 8, pipe);
+}
+
+/* The layout of new data.  Without one the data are forgotten: the layout in
+ * force was made for others. */
+static int first_launch(gpr_handle* h) {
+    const int rc = choose_launch(h);
+    if (rc != GPR_OK) forget_data(h);
+    return rc;
 }
 
 /* Device layout of a dataset: x1 | y | w | sd | x2 | x3, nd_pad floats each
@@ -648,7 +668,7 @@ static int set_data_body(gpr_handle* h, const float* x, const float* x2, const f
     kp.dw = h->ddata ? h->ddata + 2 * (size_t)nd_pad : nullptr;
     kp.dx2 = (h->ddata && three) ? h->ddata + 4 * (size_t)nd_pad : nullptr;
     kp.dx3 = (h->ddata && three) ? h->ddata + 5 * (size_t)nd_pad : nullptr;
-    return choose_launch(h);
+    return first_launch(h);
 }
 
 int gpr_set_data(gpr_handle* h, const float* x, const float* y, const float* sd, int n) {
@@ -756,7 +776,7 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
     kp.ds_order = h->dds + 2 * n_datasets;
     kp.ds_ns = h->dds_ns;
     kp.ds_ns64 = h->dds_ns64;
-    return choose_launch(h);
+    return first_launch(h);
 }
 
 static int run(gpr_handle* h, int steps, int seed);
@@ -1051,11 +1071,9 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
     if (!saved_stream)
         for (int pi = 1; pi >= 0; --pi)
             for (int ro = 0; ro <= (pi ? 0 : 1); ++ro) cands[nc++] = {4, 0, ro, 1, pi};
-    const gpr::LaunchCfg orig = h->lc;
+    const Layout orig = layout_of(h);
     float best = 1e30f;
-    gpr::LaunchCfg bestlc = orig;
-    const HmcLayout orig_hmc = h->hmc;
-    HmcLayout best_hmc = orig_hmc;
+    Layout bestl = orig;
     cudaError_t e;
     /* trial blocks leave the per-chain scales alone */
     const float saved_target = h->kp.adapt_target;
@@ -1093,7 +1111,7 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
             }
             float ms = 0.0f;
             AT_TRY(cudaEventElapsedTime(&ms, e0, e1));
-            if (ms < best) { best = ms; bestlc = h->lc; best_hmc = h->hmc; }
+            if (ms < best) { best = ms; bestl = layout_of(h); }
         }
         nc = 0;
     }
@@ -1112,11 +1130,11 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
         }
         float ms = 0.0f;
         AT_TRY(cudaEventElapsedTime(&ms, e0, e1));
-        if (ms < best) { best = ms; bestlc = h->lc; }
+        if (ms < best) { best = ms; bestl = layout_of(h); }
     }
     /* second stage: barrier period (lockstep kernel) and CTA size for the best layout */
     if (!hmc) {
-        const gpr::LaunchCfg base = bestlc;
+        const gpr::LaunchCfg base = bestl.lc;
         const int periods[3] = {1, 5, 0};
         const int wpcs[2] = {8, 4};
         for (int pi = 0; pi < (base.pipe ? 1 : 3); ++pi)
@@ -1137,20 +1155,10 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
                 }
                 float ms = 0.0f;
                 AT_TRY(cudaEventElapsedTime(&ms, e0, e1));
-                if (ms < best) { best = ms; bestlc = h->lc; }
+                if (ms < best) { best = ms; bestl = layout_of(h); }
             }
     }
-    if (!hmc) {
-        /* re-derive the chosen layout (and its scratch) rather than copying it */
-        h->stream_data = bestlc.stream ? 1 : saved_stream;
-        rc = configure_launch(h, bestlc.K, bestlc.onepass, bestlc.rolled, bestlc.lockstep, bestlc.warps_per_cta,
-                              bestlc.pipe);
-        h->stream_data = saved_stream;
-        if (rc != GPR_OK) goto done;
-    } else {
-        h->lc = bestlc;
-        h->hmc = best_hmc;
-    }
+    commit_layout(h, bestl);
     AT_TRY(cudaMemcpyAsync(h->dP, sP, cnt * sizeof(int32_t), cudaMemcpyDeviceToDevice, h->stream));
     AT_TRY(cudaMemcpyAsync(h->dC, sC, cnt * sizeof(float), cudaMemcpyDeviceToDevice, h->stream));
     AT_TRY(cudaMemcpyAsync(h->dprior, sPr, h->N * sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
@@ -1164,7 +1172,7 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
 #undef AT_TRY
 done:
     h->kp.adapt_target = saved_target;
-    if (rc != GPR_OK) { h->lc = orig; h->hmc = orig_hmc; }
+    if (rc != GPR_OK) commit_layout(h, orig);
     cudaFree(sP); cudaFree(sC); cudaFree(sPr); cudaFree(sLi); cudaFree(sSt);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);

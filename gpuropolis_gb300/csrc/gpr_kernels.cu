@@ -72,6 +72,9 @@ cudaError_t mh_occupancy(const KParams& p, const LaunchCfg& lc, int* ctas_per_sm
 cudaError_t launch_mh_block(const KParams& p, const LaunchCfg& lc, cudaStream_t st) {
     const void* f = pick_kernel(lc.K, lc.onepass, p.rng_mode, lc.rolled, lc.stream, p.nv, p.nds > 0, lc.pipe);
     if (!f) return cudaErrorInvalidValue;
+    /* more chunks than the board holds need rows in device memory */
+    if (p.part_stride < (lc.pipe ? pipe_part_stride(p.nd) : lc.K == 8 && lc.stream ? mh_part_stride(p.nd) : 0))
+        return cudaErrorInvalidValue;
     cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)lc.smem_bytes);
     if (e != cudaSuccess) return e;
     KParams pp = p;
