@@ -10,21 +10,25 @@ template __global__ void mh_block_kernel<4, false, 0, false, false, 1, false, tr
 template __global__ void mh_block_kernel<4, false, 0, false, true, 1, false, true>(const __grid_constant__ KParams p);
 template __global__ void mh_block_kernel<8, true, 0, false, false, 1, false, true>(const __grid_constant__ KParams p);
 template __global__ void mh_block_kernel<8, false, 0, false, false, 1, false, true>(const __grid_constant__ KParams p);
+template __global__ void mh_block_kernel<8, false, 0, false, true, 1, false, true>(const __grid_constant__ KParams p);
 template __global__ void mh_pipe_kernel<4, false, 0, false, false, 1, false, true>(const __grid_constant__ KParams p);
 template __global__ void mh_pipe_kernel<4, false, 0, false, true, 1, false, true>(const __grid_constant__ KParams p);
 template __global__ void mh_pipe_kernel<8, true, 0, false, false, 1, false, true>(const __grid_constant__ KParams p);
+template __global__ void mh_pipe_kernel<8, false, 0, false, true, 1, false, true>(const __grid_constant__ KParams p);
 
 static const void* pipe_prof(int K, int onepass, int rng, int stream) {
     if (rng != 0) return nullptr;
     if (K == 4 && !onepass) return stream ? (const void*)mh_pipe_kernel<4, false, 0, false, true, 1, false, true>
                                           : (const void*)mh_pipe_kernel<4, false, 0, false, false, 1, false, true>;
-    if (K == 8 && onepass && !stream) return (const void*)mh_pipe_kernel<8, true, 0, false, false, 1, false, true>;
+    if (K == 8 && stream) return onepass ? nullptr : (const void*)mh_pipe_kernel<8, false, 0, false, true, 1, false, true>;
+    if (K == 8 && onepass) return (const void*)mh_pipe_kernel<8, true, 0, false, false, 1, false, true>;
     return nullptr;
 }
 
 const void* mh_kernel_prof(int K, int onepass, int rng, int stream) {
     if (rng != 0) return nullptr;
     if (K == 4 && stream) return onepass ? nullptr : (const void*)mh_block_kernel<4, false, 0, false, true, 1, false, true>;
+    if (K == 8 && stream) return onepass ? nullptr : (const void*)mh_block_kernel<8, false, 0, false, true, 1, false, true>;
     if (stream) return nullptr;
     if (K == 4) return onepass ? (const void*)mh_block_kernel<4, true, 0, false, false, 1, false, true>
                                : (const void*)mh_block_kernel<4, false, 0, false, false, 1, false, true>;
