@@ -113,11 +113,13 @@ int cudaEventCreate(void** e) { *e = (void*)1; return OK; }
 int cudaEventDestroy(void* e) { (void)e; return OK; }
 int cudaEventRecord(void* e, void* s) { (void)e; (void)s; return OK; }
 int cudaEventSynchronize(void* e) { (void)e; return OK; }
-/* each timing a little longer than the last: the first layout tried wins */
+/* timing number fast_at is the shortest; the others are the same */
+static long fast_at, timings;
+void fake_fastest(long n) { fast_at = n; timings = 0; }
+long fake_timings(void) { return timings; }
 int cudaEventElapsedTime(float* ms, void* a, void* b) {
-    static float t = 1.0f;
     (void)a; (void)b;
-    *ms = t += 1.0f;
+    *ms = ++timings == fast_at ? 1.0f : 2.0f;
     return OK;
 }
 

@@ -40,7 +40,9 @@ def load(lib):
     g.LIB_PATH = lib
     fake = ctypes.CDLL(lib)
     fake.fake_why.restype = ctypes.c_char_p
-    fake.fake_launches.restype = fake.fake_unsafe.restype = fake.fake_clusters.restype = ctypes.c_long
+    for f in (fake.fake_launches, fake.fake_unsafe, fake.fake_clusters, fake.fake_timings):
+        f.restype = ctypes.c_long
     fake.fake_allocated.restype = ctypes.c_size_t
+    fake.fake_fastest.argtypes = [ctypes.c_long]
     fake.fake_fail.argtypes = [ctypes.c_long, ctypes.c_long]
     return g, fake
