@@ -486,24 +486,26 @@ static int configure_launch(gpr_handle* h, int K, int onepass, int rolled, int l
     auto smem_of = [&](int k, int w, int st) {
         return pipe ? gpr::pipe_smem_bytes(kp, k, w, st) : gpr::mh_smem_bytes(kp, k, w, st, rolled);
     };
-    lc.stream = h->stream_data || (K == 8 && kp.nv == 3) || smem_of(K, wpc0, 0) > 227 * 1024;
-    if (lc.stream) {
-        if (kp.nds > 0 || rolled) K = 4;
-        onepass = 0;
-    }
     lc.K = K;
     lc.onepass = onepass;
     lc.rolled = rolled;
     lc.lockstep = lockstep;
     lc.pipe = pipe;
+    lc.stream = h->stream_data || (K == 8 && kp.nv == 3);
+    lc.stream = lc.stream || smem_of(K, wpc0, 0) > gpr::mh_smem_limit(kp, lc);
+    if (lc.stream) {
+        if (kp.nds > 0 || rolled) lc.K = 4;
+        lc.onepass = 0;
+    }
+    const size_t limit = gpr::mh_smem_limit(kp, lc);
     int wpc = wpc0;
     size_t smem = smem_of(lc.K, wpc, lc.stream);
-    while (smem > 227 * 1024 && wpc > 1) {
+    while (smem > limit && wpc > 1) {
         wpc /= 2;
         smem = smem_of(lc.K, wpc, lc.stream);
     }
     if (kp.nds > 0) wpc = batched_wpc(kp, wpc, pipe);
-    if (smem > 227 * 1024)
+    if (smem > limit)
         return fail(h, GPR_ERR_ARG, "programs of length %d do not fit in shared memory", kp.PL);
     lc.warps_per_cta = wpc;
     lc.smem_bytes = smem;

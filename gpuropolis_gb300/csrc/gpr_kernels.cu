@@ -61,6 +61,13 @@ void fill_lcg_jump_table(KParams& p) {
     }
 }
 
+size_t mh_smem_limit(const KParams& p, const LaunchCfg& lc) {
+    const void* f = pick_kernel(lc.K, lc.onepass, p.rng_mode, lc.rolled, lc.stream, p.nv, p.nds > 0, lc.pipe);
+    cudaFuncAttributes a = {};
+    if (f && cudaFuncGetAttributes(&a, f) != cudaSuccess) (void)cudaGetLastError();   /* the launch will say */
+    return GPR_CTA_SMEM - a.sharedSizeBytes;
+}
+
 cudaError_t mh_occupancy(const KParams& p, const LaunchCfg& lc, int* ctas_per_sm) {
     const void* f = pick_kernel(lc.K, lc.onepass, p.rng_mode, lc.rolled, lc.stream, p.nv, p.nds > 0, lc.pipe);
     if (!f) return cudaErrorInvalidValue;

@@ -175,6 +175,10 @@ cudaError_t launch_mh_block_prof(const KParams& p, const LaunchCfg& lc, cudaStre
 const void* mh_kernel_prof(int K, int onepass, int rng, int stream);
 const void* prof_kernel(const LaunchCfg& lc);   /* the LCG phase-timed build of lc, or nullptr */
 cudaError_t mh_occupancy(const KParams& p, const LaunchCfg& lc, int* ctas_per_sm);
+/* Dynamic shared memory that a CTA of lc's kernel can have: what its static
+ * variables leave (no limit of its own where lc has no kernel). */
+#define GPR_CTA_SMEM ((size_t)227 * 1024)
+size_t mh_smem_limit(const KParams& p, const LaunchCfg& lc);
 
 /* Diagnostics: evaluate every chain's program at nx points, and report the
  * compiled length / node count (used by the parity tests). */

@@ -9,7 +9,7 @@
 #include <string.h>
 
 typedef struct { unsigned x, y, z; } dim3_t;
-enum { OK = 0, ERR_MEMORY = 2, ERR_CONFIG = 9, ERR_UNSUPPORTED = 801 };
+enum { OK = 0, ERR_VALUE = 1, ERR_MEMORY = 2, ERR_CONFIG = 9, ERR_UNSUPPORTED = 801 };
 
 #define MAX_BLOCKS 4096
 static struct { char* p; size_t n; } blocks[MAX_BLOCKS];
@@ -95,10 +95,17 @@ int cudaDeviceGetAttribute(int* v, int a, int d) {
     *v = a == 16 ? 152 : a == 81 ? 233472 : 0;   /* SMs; shared memory per SM */
     return OK;
 }
-int cudaFuncSetAttribute(const void* f, int a, int v) { (void)f; (void)a; (void)v; return OK; }
+/* every kernel has 6 KB of static shared memory, as the block kernels about have */
+#define STATIC_SMEM 6144
+#define CTA_SMEM (227 * 1024)
+int cudaFuncGetAttributes(size_t* a, const void* f) { (void)f; a[0] = STATIC_SMEM; return OK; }
+int cudaFuncSetAttribute(const void* f, int a, int v) {
+    (void)f;
+    return a == 8 && v + STATIC_SMEM > CTA_SMEM ? err(ERR_VALUE) : OK;   /* 8: dynamic shared memory */
+}
 int cudaOccupancyMaxActiveBlocksPerMultiprocessor(int* n, const void* f, int threads, size_t smem) {
     (void)f;
-    const int by_smem = (int)(233472 / (smem + 1024)), by_threads = 768 / threads;
+    const int by_smem = (int)(233472 / (smem + STATIC_SMEM + 1024)), by_threads = 768 / threads;
     *n = by_smem < by_threads ? by_smem : by_threads;
     return OK;
 }
