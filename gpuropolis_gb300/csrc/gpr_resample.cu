@@ -232,11 +232,15 @@ __global__ void __launch_bounds__(256) below_kernel(const double* prior, const d
 }
 
 #define GPR_RD_THREADS 256
-#define GPR_RD_CHAINS 32     /* chains a CTA re-draws, one per lane */
 
-/* Shared memory of a CTA that keeps `draws` draws per chain (a multiple of 32). */
-__host__ __device__ __forceinline__ size_t redraw_smem_bytes(int PL, int draws) {
-    return (size_t)GPR_RD_CHAINS * ((size_t)draws * 4 + (size_t)(draws / 32) * 12 + (size_t)PL * 4);
+/* Where draw q of a chain is kept, in rows of CH.  With fewer than 32 chains a
+ * row is left out after every 32 draws, so that the threads of a warp that work
+ * on different words of them meet different banks. */
+__host__ __device__ __forceinline__ constexpr int redraw_row(int CH, int q) { return CH < 32 ? q + (q >> 5) : q; }
+/* Shared memory of a CTA that re-draws CH chains and keeps `draws` draws of
+ * each (a multiple of 32). */
+__host__ __device__ __forceinline__ size_t redraw_smem_bytes(int CH, int PL, int draws) {
+    return (size_t)CH * ((size_t)redraw_row(CH, draws) * 4 + (size_t)(draws / 32) * 12 + (size_t)PL * 4);
 }
 
 /* A draw as the CTA keeps it: what it would be as a uniform's integer, as an
@@ -258,22 +262,24 @@ __host__ __device__ __forceinline__ size_t redraw_smem_bytes(int PL, int draws) 
  * random_int rejects (one op draw in n_ops, one order draw in nine, one
  * uniform's in 4,400), so which draw belongs to what is only known one after
  * the other; the draws themselves (counter-based, 90 instructions per four)
- * and the normals (about 95 each) are not serial.  A CTA takes 32 chains (lane =
- * chain) in phases:
- *   1. all warps make the first `draws` draws of every chain and, 32 at a time,
+ * and the normals (about 95 each) are not serial.  A CTA takes CH chains, its
+ * threads in groups of one per chain, in phases:
+ *   1. all groups make the first `draws` draws of every chain and, 32 at a time,
  *      the bits that say which random_int would take as an op, as an order, and
  *      not as a uniform;
- *   2. all warps, a word of those bits each: the ops' positions by their rank,
+ *   2. all groups, a word of those bits each: the ops' positions by their rank,
  *      and for every draw the distance to the order that follows if it is one;
  *   3. one thread per chain follows those distances and notes each constant's
  *      position, while the other warps write the ops;
- *   4. all warps make the constants.
+ *   4. all groups make the constants.
  * A chain that needs more draws than were made is drawn one after the other by
  * its own thread.
  * 65,536 of 131,072 chains of 63 nodes: 89 us.  One thread per chain for
  * all of it: 195 us (long dependent sequences in few warps, and a Philox block
  * issued by the warp whenever one of its threads ran out of draws).  Phases 2
- * and 3 as one thread's walk over the bits: 122 us (the other warps wait). */
+ * and 3 as one thread's walk over the bits: 122 us (the other warps wait).
+ * CH: see launch_redraw. */
+template <int CH>
 __global__ void __launch_bounds__(GPR_RD_THREADS) redraw_kernel(const __grid_constant__ KParams p, const int* list,
                                                                 const int* n_list, uint32_t seed,
                                                                 uint32_t chain_offset, Magic mag_ops1,
@@ -283,37 +289,39 @@ __global__ void __launch_bounds__(GPR_RD_THREADS) redraw_kernel(const __grid_con
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float s_pow10[8];
     __shared__ int32_t s_map[32];
-    __shared__ int s_start[GPR_RD_CHAINS];                     /* first draw after the ops (-1: too few draws) */
-    __shared__ int s_slow[GPR_RD_CHAINS];
+    __shared__ int s_start[CH];                                /* first draw after the ops (-1: too few draws) */
+    __shared__ int s_slow[CH];
     const int PL = p.PL, nw = draws / 32;
-    uint32_t* s_draw = (uint32_t*)smem + (threadIdx.x & 31);   /* [draws][32], this lane's column */
-    uint32_t* s_opbit = s_draw + draws * GPR_RD_CHAINS;        /* [draws / 32][32]: taken as an op ... */
-    uint32_t* s_orbit = s_opbit + nw * GPR_RD_CHAINS;          /* ... as an order ... */
-    uint32_t* s_unbit = s_orbit + nw * GPR_RD_CHAINS;          /* ... rejected as a uniform */
-    uint16_t* s_oppos = (uint16_t*)((uint32_t*)smem + (draws + 3 * nw) * GPR_RD_CHAINS) + (threadIdx.x & 31);   /* [PL][32] */
-    uint16_t* s_cpos = s_oppos + PL * GPR_RD_CHAINS;           /* [PL][32] */
+    const int tid = (int)threadIdx.x, c = tid % CH, group = tid / CH, groups = GPR_RD_THREADS / CH;
+    const int rows = redraw_row(CH, draws);
+    uint32_t* s_draw = (uint32_t*)smem + c;                    /* [rows][CH], this chain's column */
+    uint32_t* s_opbit = s_draw + rows * CH;                    /* [draws / 32][CH]: taken as an op ... */
+    uint32_t* s_orbit = s_opbit + nw * CH;                     /* ... as an order ... */
+    uint32_t* s_unbit = s_orbit + nw * CH;                     /* ... rejected as a uniform */
+    uint16_t* s_oppos = (uint16_t*)((uint32_t*)smem + (rows + 3 * nw) * CH) + c;   /* [PL][CH] */
+    uint16_t* s_cpos = s_oppos + PL * CH;                      /* [PL][CH] */
+    auto draw = [&](int q) -> uint32_t& { return s_draw[redraw_row(CH, q) * CH]; };
     const int n = *n_list;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = GPR_RD_THREADS / 32;
-    const int first = blockIdx.x * GPR_RD_CHAINS;
+    const int first = blockIdx.x * CH;
     if (first >= n) return;
-    if (threadIdx.x < 8) s_pow10[threadIdx.x] = gpr_pow10_order((int)threadIdx.x - 4);
-    if (warp == 1) s_map[lane] = p.opmap[lane];
-    if (warp == 2) s_start[lane] = -1;
-    /* lanes past the list's end follow its last chain and write nothing */
-    const bool live = first + lane < n;
-    const int chain = list[min(first + lane, n - 1)];
+    if (tid < 8) s_pow10[tid] = gpr_pow10_order(tid - 4);
+    if (tid >= 32 && tid < 64) s_map[tid - 32] = p.opmap[tid - 32];
+    if (tid >= 64 && tid < 64 + CH) s_start[tid - 64] = -1;
+    /* threads past the list's end follow its last chain and write nothing */
+    const bool live = first + c < n;
+    const int chain = list[min(first + c, n - 1)];
     const uint32_t key1 = ((uint32_t)chain + chain_offset) | 0x80000000u;
 #pragma unroll 1
-    for (int w = warp; w < nw; w += nwarps) {
+    for (int w = group; w < nw; w += groups) {
         uint32_t ob = 0u, rb = 0u, ub = 0u;
 #pragma unroll 2
         for (int b = 0; b < 8; ++b) {
-            uint32_t c[4] = {(uint32_t)(8 * w + b), 0u, 0u, 0u};
-            gpr_philox4x32_10(c, seed, key1);
+            uint32_t r[4] = {(uint32_t)(8 * w + b), 0u, 0u, 0u};
+            gpr_philox4x32_10(r, seed, key1);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const uint32_t x = c[j] >> 1;
-                s_draw[(32 * w + 4 * b + j) * GPR_RD_CHAINS] =
+                const uint32_t x = r[j] >> 1;
+                draw(32 * w + 4 * b + j) =
                     (magic_div(x, p.mag_1e6) & 0xfffffu) | ((magic_div(x, mag_order) & 7u) << 20) |
                     ((magic_div(x, mag_ops1) & 31u) << 23);
                 ob |= (x < op_below ? 1u : 0u) << (4 * b + j);
@@ -321,48 +329,48 @@ __global__ void __launch_bounds__(GPR_RD_THREADS) redraw_kernel(const __grid_con
                 ub |= (x < uniform_below ? 0u : 1u) << (4 * b + j);
             }
         }
-        s_opbit[w * GPR_RD_CHAINS] = ob;
-        s_orbit[w * GPR_RD_CHAINS] = rb;
-        s_unbit[w * GPR_RD_CHAINS] = ub;
+        s_opbit[w * CH] = ob;
+        s_orbit[w * CH] = rb;
+        s_unbit[w * CH] = ub;
     }
     __syncthreads();
 #pragma unroll 1
-    for (int w = warp; w < nw; w += nwarps) {
+    for (int w = group; w < nw; w += groups) {
         int rank = 0;
-        for (int v = 0; v < w; ++v) rank += __popc(s_opbit[v * GPR_RD_CHAINS]);
-        uint32_t m = s_opbit[w * GPR_RD_CHAINS];
+        for (int v = 0; v < w; ++v) rank += __popc(s_opbit[v * CH]);
+        uint32_t m = s_opbit[w * CH];
         for (; m && rank < PL; ++rank, m &= m - 1u) {
             const int pos = 32 * w + __ffs(m) - 1;
-            s_oppos[rank * GPR_RD_CHAINS] = (uint16_t)pos;
-            if (rank == PL - 1) s_start[lane] = pos + 1;
+            s_oppos[rank * CH] = (uint16_t)pos;
+            if (rank == PL - 1) s_start[c] = pos + 1;
         }
         /* an order, two uniforms, and on to the next order */
-        const uint32_t r0 = s_orbit[w * GPR_RD_CHAINS], r1 = w + 1 < nw ? s_orbit[(w + 1) * GPR_RD_CHAINS] : 0u;
-        const uint32_t u0 = s_unbit[w * GPR_RD_CHAINS], u1 = w + 1 < nw ? s_unbit[(w + 1) * GPR_RD_CHAINS] : ~0u;
+        const uint32_t r0 = s_orbit[w * CH], r1 = w + 1 < nw ? s_orbit[(w + 1) * CH] : 0u;
+        const uint32_t u0 = s_unbit[w * CH], u1 = w + 1 < nw ? s_unbit[(w + 1) * CH] : ~0u;
 #pragma unroll
         for (int b = 0; b < 32; ++b) {
             const uint32_t next = b + 3 < 32 ? __funnelshift_r(r0, r1, (b + 3) & 31) : r1 >> ((b + 3) & 31);
             const uint32_t uni = b + 1 < 32 ? __funnelshift_r(u0, u1, (b + 1) & 31) : u1;
             const uint32_t step = (uint32_t)__ffs(next) + 2u;
             const bool far = next == 0u || step >= GPR_RD_FAR || (uni & 3u);
-            s_draw[(32 * w + b) * GPR_RD_CHAINS] |= (far ? GPR_RD_FAR : step) << 28;
+            draw(32 * w + b) |= (far ? GPR_RD_FAR : step) << 28;
         }
     }
     __syncthreads();
     auto find = [&](const uint32_t* bits, int q, uint32_t flip) {   /* the first draw from q on whose bit is set */
-        while (q < draws && !(((bits[(q >> 5) * GPR_RD_CHAINS] ^ flip) >> (q & 31)) & 1u)) ++q;
+        while (q < draws && !(((bits[(q >> 5) * CH] ^ flip) >> (q & 31)) & 1u)) ++q;
         return q;
     };
     const size_t N = (size_t)p.N;
-    if (warp == 0) {
-        int pos = s_start[lane];
+    if (tid < CH) {
+        int pos = s_start[c];
         bool slow = pos < 0;
         if (!slow) pos = find(s_orbit, pos, 0u);
 #pragma unroll 1
         for (int node = 0; node < PL && !slow; ++node) {
             if (pos + 2 >= draws) { slow = true; break; }
-            s_cpos[node * GPR_RD_CHAINS] = (uint16_t)pos;
-            const uint32_t step = GPR_RD_STEP(s_draw[pos * GPR_RD_CHAINS]);
+            s_cpos[node * CH] = (uint16_t)pos;
+            const uint32_t step = GPR_RD_STEP(draw(pos));
             if (step != GPR_RD_FAR) {
                 pos += (int)step;
             } else {
@@ -371,28 +379,28 @@ __global__ void __launch_bounds__(GPR_RD_THREADS) redraw_kernel(const __grid_con
                 pos = find(s_orbit, pos, 0u);
             }
         }
-        s_slow[lane] = slow;
-    } else if (live && s_start[lane] >= 0) {
+        s_slow[c] = slow;
+    } else if (tid >= 32 && live && s_start[c] >= 0) {
 #pragma unroll 4
-        for (int i = warp - 1; i < PL; i += nwarps - 1)
-            p.P[(size_t)i * N + chain] = s_map[GPR_RD_OP(s_draw[s_oppos[i * GPR_RD_CHAINS] * GPR_RD_CHAINS])];
+        for (int i = group - 32 / CH; i < PL; i += groups - 32 / CH)
+            p.P[(size_t)i * N + chain] = s_map[GPR_RD_OP(draw(s_oppos[i * CH]))];
     }
     __syncthreads();
-    const bool fast = live && !s_slow[lane];
+    const bool fast = live && !s_slow[c];
 #pragma unroll 1
-    for (int i = warp; i < PL; i += nwarps) {
+    for (int i = group; i < PL; i += groups) {
         if (!fast) continue;
-        const int c = s_cpos[i * GPR_RD_CHAINS];
-        const uint32_t w = s_draw[c * GPR_RD_CHAINS];
-        int qu = c + 1, qv = c + 2;
+        const int q = s_cpos[i * CH];
+        const uint32_t w = draw(q);
+        int qu = q + 1, qv = q + 2;
         if (GPR_RD_STEP(w) == GPR_RD_FAR) { qu = find(s_unbit, qu, ~0u); qv = find(s_unbit, qu + 1, ~0u); }
-        const float u = gpr_rng_k_over_1e6((int)GPR_RD_UNIFORM(s_draw[qu * GPR_RD_CHAINS]));
-        const float v = gpr_rng_k_over_1e6((int)GPR_RD_UNIFORM(s_draw[qv * GPR_RD_CHAINS]));
+        const float u = gpr_rng_k_over_1e6((int)GPR_RD_UNIFORM(draw(qu)));
+        const float v = gpr_rng_k_over_1e6((int)GPR_RD_UNIFORM(draw(qv)));
         const float a = __fsqrt_rn(__fmul_rn(-2.0f, gpr_rng_logf(u)));
         const float z = __fmul_rn(a, gpr_rng_sinf(gpr_rng_twopi_times(v)));
         p.C[(size_t)i * N + chain] = __fmul_rn(s_pow10[GPR_RD_ORDER(w)], z);
     }
-    if (warp == 0 && live && !fast) {
+    if (tid < CH && live && !fast) {
         Rng r;
         r.s = 0u; r.key0 = seed; r.key1 = key1; r.blk = 0xffffffffu; r.drawn = 0u;
         r.w0 = r.w1 = r.w2 = r.w3 = 0u;
@@ -451,6 +459,14 @@ cudaError_t launch_select(const KParams& p, int rank, unsigned long long* keys, 
     return cudaLaunchKernelEx(&cfg, select_rank_kernel, p.prior, p.lik, keys, n, rank, out, zero, host);
 }
 
+/* Chains per CTA (CH): the most of 32, 16 and 8 whose draws leave room for three
+ * CTAs per SM, whose phases then overlap.  131,072 chains, 95% of them re-drawn,
+ * 8 ops: 127 nodes 446 us with 32 chains (98 KB), 410 with 16; 255 nodes 1,359
+ * with 32 (186 KB), 1,118 with 16 and 1,028 with 8, 1,086 with a thread per chain
+ * (selection over one CTA included).  Two ops, 255 nodes: 14.2 ms where 200 KB for
+ * 32 chains cut their draws short, 1.30 now, 1.43 with a thread per chain. */
+#define GPR_RD_SMEM (72 * 1024)
+
 cudaError_t launch_redraw(const KParams& p, const unsigned long long* sel_key, int seg_len, int map_delta,
                           double delta, uint32_t seed, Magic mag_ops1, Magic mag_order, int* list, int* n_redrawn,
                           cudaStream_t st, uint32_t chain_offset) {
@@ -460,20 +476,21 @@ cudaError_t launch_redraw(const KParams& p, const unsigned long long* sel_key, i
     if (e != cudaSuccess) return e;
     /* Draws per chain kept in shared memory: the mean and eight standard
      * deviations (an op takes a draw in n_ops - 1 of n_ops cases, an order one in
-     * 8 of 9), as far as a CTA's shared memory goes. */
+     * 8 of 9): at most 1,536, of 255 nodes and two ops. */
     const double q = 1.0 / p.nops, mean = p.PL * (1.0 / (1.0 - q) + 2.0 + 9.0 / 8.0),
                  sd = sqrt(p.PL * (q / ((1.0 - q) * (1.0 - q)) + 9.0 / 64.0));
-    int draws = ((int)(mean + 8.0 * sd + 4.0) + 31) / 32 * 32;
-    while (redraw_smem_bytes(p.PL, draws) > 200 * 1024) draws -= 32;
-    const size_t smem = redraw_smem_bytes(p.PL, draws);
-    e = cudaFuncSetAttribute((const void*)redraw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+    const int draws = ((int)(mean + 8.0 * sd + 4.0) + 31) / 32 * 32;
     /* x / d < n  <=>  x < n d, d the divisor of random_int(n) */
     const uint32_t op_below = (uint32_t)(p.nops - 1) * (2147483647u / (uint32_t)p.nops),
                    order_below = 8u * (2147483647u / 9u), uniform_below = 1000000u * (2147483647u / 1000001u);
-    redraw_kernel<<<(p.N + GPR_RD_CHAINS - 1) / GPR_RD_CHAINS, GPR_RD_THREADS, smem, st>>>(
-        p, list, n_redrawn, seed, chain_offset, mag_ops1, mag_order, op_below, order_below, uniform_below,
-        draws);
+    int CH = 32;
+    while (CH > 8 && redraw_smem_bytes(CH, p.PL, draws) > GPR_RD_SMEM) CH /= 2;
+    const size_t smem = redraw_smem_bytes(CH, p.PL, draws);
+    const auto f = CH == 32 ? redraw_kernel<32> : CH == 16 ? redraw_kernel<16> : redraw_kernel<8>;
+    e = cudaFuncSetAttribute((const void*)f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    f<<<(p.N + CH - 1) / CH, GPR_RD_THREADS, smem, st>>>(p, list, n_redrawn, seed, chain_offset, mag_ops1, mag_order,
+                                                         op_below, order_below, uniform_below, draws);
     return cudaGetLastError();
 }
 
