@@ -441,22 +441,31 @@ cudaError_t launch_select(const KParams& p, int rank, unsigned long long* keys, 
     /* One CTA up to GPR_SEL_ONE keys (four per thread): a round over them takes
      * less than a cluster barrier, and a batched handle's segments (hundreds of
      * them, 15 us for 256 of 512 keys) fill the device by themselves. */
-    const int ncta = n > GPR_SEL_ONE ? GPR_SEL_CLUSTER : 1;
+    int ncta = n > GPR_SEL_ONE ? GPR_SEL_CLUSTER : 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)segments * ncta);
     cfg.blockDim = dim3((unsigned)std::min(GPR_SEL_THREADS, (n + 31) / 32 * 32));
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ncta;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     cudaError_t e = cudaFuncSetAttribute((const void*)select_rank_kernel,
                                          cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, select_rank_kernel, p.prior, p.lik, keys, n, rank, out, zero, host);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        ncta = 1;
+    }
+    /* Where a cluster of that size cannot be resident (it is beyond the portable
+     * eight) the launch says so, and one CTA selects. */
+    for (;; ncta = 1) {
+        cfg.gridDim = dim3((unsigned)segments * ncta);
+        attr[0].val.clusterDim.x = ncta;
+        e = cudaLaunchKernelEx(&cfg, select_rank_kernel, p.prior, p.lik, keys, n, rank, out, zero, host);
+        if (e == cudaSuccess || ncta == 1) return e;
+        (void)cudaGetLastError();
+    }
 }
 
 /* Chains per CTA (CH): the most of 32, 16 and 8 whose draws leave room for three
