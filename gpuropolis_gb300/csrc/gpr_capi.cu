@@ -700,12 +700,12 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
                                        h->N, n_datasets);
     const int cpd = h->N / n_datasets;
     const bool three = h->kp.nv == 3;
-    long long total = 0, maxn = 0, npad = 0, nchunk = 0;
+    long long total = 0, maxn = 0, npad = 0, packed = 0;
     for (int d = 0; d < n_datasets; ++d) {
         if (sizes[d] < 0) return fail(h, GPR_ERR_ARG, "sizes[%d] = %d is negative", d, sizes[d]);
         total += sizes[d];
         npad += (sizes[d] + 3) & ~3;
-        nchunk += ((long long)sizes[d] + GPR_CHUNK_POINTS - 1) / GPR_CHUNK_POINTS;
+        packed += GPR_PACKED_POINTS(sizes[d]);
         if (sizes[d] > maxn) maxn = sizes[d];
     }
     if (npad > (1ll << 30)) return fail(h, GPR_ERR_ARG, "batched data too large");
@@ -715,8 +715,8 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
         if (!(sd[i] > 0.0f)) return fail(h, GPR_ERR_ARG, "sd[%lld] = %g is not > 0", i, (double)sd[i]);
     CUDA_TRY(h, cudaSetDevice(h->device));
     drop_graph(h);
-    const size_t T = (size_t)nchunk * GPR_CHUNK_POINTS;   /* npad <= 2^30: at most 2^28 chunks */
-    std::vector<float> host((three ? 6 : 4) * T + 4, 0.0f);
+    const size_t T = (size_t)packed;   /* at most 4 npad: 2^32 */
+    std::vector<float> host((three ? 6 : 4) * T + GPR_CHUNK_POINTS, 0.0f);
     std::vector<int> meta(3 * (size_t)n_datasets);
     std::vector<float> ns(2 * (size_t)n_datasets);
     std::vector<double> ns64((size_t)n_datasets);
@@ -724,7 +724,7 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
     const int we = weight_exponent(sd, (size_t)total);
     size_t off = 0, src = 0;
     for (int d = 0; d < n_datasets; ++d) {
-        meta[d] = (int)(off / GPR_CHUNK_POINTS);
+        meta[d] = (int)(off / 4);
         meta[n_datasets + d] = sizes[d];
         double normsum = 0.0;
         for (int i = 0; i < sizes[d]; ++i, ++src) {
@@ -740,7 +740,7 @@ static int set_batched_body(gpr_handle* h, int n_datasets, const int* sizes, con
         const double nsd = normsum * 0x1p-64;
         ns[2 * d] = (float)nsd;
         ns[2 * d + 1] = (float)(nsd - (double)ns[2 * d]);
-        off += (size_t)GPR_PAD_POINTS(sizes[d]);
+        off += (size_t)GPR_PACKED_POINTS(sizes[d]);
     }
     /* datasets claimed largest first, so that uneven sizes balance across the grid */
     std::vector<int> order(n_datasets);

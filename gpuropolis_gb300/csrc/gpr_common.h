@@ -181,6 +181,12 @@ enum gpr_phase {
  * that a lane's four points are one 16-byte load. */
 #define GPR_CHUNK_POINTS 128
 #define GPR_PAD_POINTS(n) (((n) + GPR_CHUNK_POINTS - 1) / GPR_CHUNK_POINTS * GPR_CHUNK_POINTS)
+/* The same for one of many datasets behind each other: of its last chunk only
+ * the lanes that have a point, four floats each, so that datasets of a few points
+ * take at most four times their size.  A reader of that chunk's other lanes meets
+ * the next dataset; after the last one there is a chunk more. */
+#define GPR_PACKED_POINTS(n) ((n) / GPR_CHUNK_POINTS * GPR_CHUNK_POINTS + \
+                              4 * ((n) % GPR_CHUNK_POINTS < 32 ? (n) % GPR_CHUNK_POINTS : 32))
 /* Where point i of a dataset is in its arrays. */
 #define GPR_POINT_SLOT(i) (((i) & ~127) | (((i) & 31) << 2) | (((i) >> 5) & 3))
 

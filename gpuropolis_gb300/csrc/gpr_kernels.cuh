@@ -38,8 +38,8 @@ struct KParams {
     const float* dx2;  /* multivariate data: the second and third input variables */
     const float* dx3;
     int nv;            /* input variables: 1, or 3 for x1, x2, x3 (0 reads as 1) */
-    /* batched data (nds > 0): dataset d is the ds_n[d] points from chunk ds_off[d]
-     * of the arrays on, with normalising sum ds_ns[2d],
+    /* batched data (nds > 0): dataset d is the ds_n[d] points from element
+     * 4 ds_off[d] of the arrays on (GPR_PACKED_POINTS), with normalising sum ds_ns[2d],
      * ds_ns[2d+1] (2^-64 scale, double-float); chain c belongs to dataset
      * c / chains_per_ds; chain groups are claimed dataset by dataset in the
      * order ds_order (largest first); nd / nd_pad then give the largest */
