@@ -513,7 +513,7 @@ __device__ __forceinline__ void backward_tape(const uint2* __restrict__ prog, in
                 GPR_EACH adj[k] = adj_mul(adj[k], c);
                 continue;
             }
-            const bool takes = src == SRC_C || src == SRC_POP;
+            const bool takes = GW_AUX(w) != GW_NONE;   /* the operand has a share: popped, or a constant of the program */
             float av[K];          /* the operand's share per point */
             if (bop == BOP_SUB) {
                 GPR_EACH av[k] = -adj[k];
