@@ -492,12 +492,13 @@ static int configure_launch(gpr_handle* h, int K, int onepass, int rolled, int l
     lc.lockstep = lockstep;
     lc.pipe = pipe;
     lc.stream = h->stream_data || (K == 8 && kp.nv == 3);
-    lc.stream = lc.stream || smem_of(K, wpc0, 0) > gpr::mh_smem_limit(kp, lc);
-    if (lc.stream) {
+    size_t limit = lc.stream ? 0 : gpr::mh_smem_limit(kp, lc);
+    if (lc.stream || smem_of(K, wpc0, 0) > limit) {
+        lc.stream = 1;
         if (kp.nds > 0 || rolled) lc.K = 4;
         lc.onepass = 0;
+        limit = gpr::mh_smem_limit(kp, lc);
     }
-    const size_t limit = gpr::mh_smem_limit(kp, lc);
     int wpc = wpc0;
     size_t smem = smem_of(lc.K, wpc, lc.stream);
     while (smem > limit && wpc > 1) {
@@ -582,10 +583,10 @@ static int choose_launch(gpr_handle* h) {
         return configure_streamed(h, 8, 0);
     int rc = configure_launch(h, 4, onepass, 0, 1, 8, pipe);
     if (rc != GPR_OK || hmc || h->lc.stream || onepass || kp.nd <= 0) return rc;
-    const int staged = h->lc.ctas;
+    const Layout staged = layout_of(h);
     rc = configure_streamed(h, 4, pipe);
-    if (rc == GPR_OK && h->lc.ctas > staged) return rc;
-    return configure_launch(h, 4, 0, 0, 1, 8, pipe);
+    if (rc != GPR_OK || h->lc.ctas <= staged.lc.ctas) commit_layout(h, staged);
+    return GPR_OK;
 }
 
 /* The layout of new data.  Without one the data are forgotten: the layout in
