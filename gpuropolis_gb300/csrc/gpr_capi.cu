@@ -399,13 +399,16 @@ static int batched_wpc(const gpr::KParams& kp, int wpc, int pipe = 0) {
  * the shared-memory carveout, which leaves the rest of the SM's L1 to what is
  * spilled.
  *
- * stream_mode -1: the data are staged up to two passes and read from device
- * memory beyond.  Staged / streamed, 65,536 chains: 128 points 0.92-0.98 (fixed
- * programs and random ones of one variable; 1.06 random ones of three), 300
- * points 0.96-1.18, 1,024 points 0.98-1.34, 2,048 points 1.10-1.48.  Streamed as
- * well when asked, for batched data (each warp reads its own chain's dataset)
- * and where staging does not fit. */
-#define GPR_HMC_STAGED_POINTS (2 * GPR_CHUNK_POINTS)
+ * stream_mode -1: the data are staged up to 3 KB, 6 KB with G = 2, and read from
+ * device memory beyond.  Staged / streamed, 65,536 chains: G = 1, 128 points of one
+ * variable 0.96 (fixed programs) and 0.98 (random), 300 points 1.01 and 1.00, 1,024
+ * points 1.15 and 1.13; three variables, 128 points 0.96 and 1.06, 300 points 1.04
+ * and 1.18.  G = 2: one variable, 128 points 0.92 and 0.99, 300 points 0.96 and
+ * 0.99, 600 points 0.99 for both, 2,048 points 1.13 and 1.10; three variables, 300
+ * points 1.03 and 0.99, 600 points 1.09 and 1.01.  Streamed as well when asked, for
+ * batched data (each warp reads its own chain's dataset) and where staging does not
+ * fit. */
+#define GPR_HMC_STAGED_BYTES 3072
 
 static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int stream_mode = -1, int G = 0) {
     if (wpc0 < 1 || wpc0 > 8) wpc0 = 4;
@@ -417,7 +420,9 @@ static int configure_hmc(gpr_handle* h, int wpc0 = 4, int ctas_per_sm = 0, int s
     gpr::LaunchCfg lc;
     lc.K = 4 * g; lc.onepass = 0; lc.rolled = 0; lc.lockstep = 0; lc.carveout = 0; lc.pipe = 0;
     lc.stream = h->stream_data || kp.nds > 0 || gpr::grad_smem_bytes(kp, g, wpc0, 0) > 227 * 1024 ||
-                (stream_mode < 0 ? kp.nd > GPR_HMC_STAGED_POINTS : stream_mode > 0);
+                (stream_mode < 0 ? gpr::grad_smem_bytes(kp, g, 1, 0) - gpr::grad_smem_bytes(kp, g, 1, 1) >
+                                   (size_t)g * GPR_HMC_STAGED_BYTES
+                             : stream_mode > 0);
     int wpc = wpc0;
     size_t smem = gpr::grad_smem_bytes(kp, g, wpc, lc.stream);
     while (smem > 227 * 1024 && wpc > 1) smem = gpr::grad_smem_bytes(kp, g, wpc /= 2, lc.stream);

@@ -27,15 +27,15 @@ bool grad_supported(const KParams& p) { return p.max_instr <= 258 && p.PL <= 127
  * 14.5 and 19.3 ms, 1,024 points 43.9 and 68.6 ms.
  * With at most 16 warps per SM for all chains, those of G = 2 have more registers
  * at no cost (2,048 chains of three variables, 4,096 points: 24.5 and 17.9 ms);
- * up to 32 it is as fast or faster from two passes on (4,096 chains: 1,024
- * points 9.1 and 6.9 ms, 384 points 3.9 and 4.7 ms); up to 48 from four (6,000
- * chains: 1,024 points 10.5 and 9.4, 384 points 4.9 and 6.5 ms). */
+ * up to 32 it is as fast or faster (4,096 chains: 1,024 points 9.1 and 6.9 ms), but
+ * for three passes, which take two sweeps (384 points 3.9 and 4.7 ms); up to 48
+ * from four passes on (6,000 chains, 1,024 points: 10.5 and 9.4 ms). */
 int hmc_passes(const KParams& p, int sms) {
     const int passes = (p.nd + GPR_CHUNK_POINTS - 1) / GPR_CHUNK_POINTS;
     if (p.N <= 16 * sms) return 2;
     if (passes <= 1) return 1;
-    if (p.struct_every == 0 || p.N <= 32 * sms) return 2;
-    return p.N <= 48 * sms && passes >= 4 ? 2 : 1;
+    if (p.struct_every == 0) return 2;
+    return p.N <= 32 * sms && passes != 3 || p.N <= 48 * sms && passes > 3 ? 2 : 1;
 }
 
 template <int MAXR>
