@@ -79,7 +79,7 @@ METRIC = "MH chain-steps/s & point-evals/s (1 GB300); ESS/s gradient vs random-w
 # DRAM bytes (read + write) of one mh_block_kernel launch of the plain-mh-131k workload, taken
 # from an ncu capture of that launch (dram__bytes_read.sum + dram__bytes_write.sum), not measured
 # in this run: the chain state read and written once; the dataset lives in shared memory.
-MH_LAUNCH_DRAM_BYTES = 113.43e6
+MH_LAUNCH_DRAM_BYTES = 100.55e6
 MH_LAUNCH_DRAM_SOURCE = "ncu capture of one launch (dram__bytes_read.sum + dram__bytes_write.sum), not this run"
 
 

@@ -62,8 +62,8 @@ static cudaError_t launch_grad(const KParams& p, int G, int wpc, double* grad, d
  * from four passes on both run: G = 2 lists the programs with a long op for G = 1
  * (1.00 and 3.01 ms).  With fewer, the second compile costs more than G = 2 gives:
  * G = 1 for all (300 points: 0.59 and 1.70 ms, listed 0.67 and 1.87).  Up to
- * 32 chains per SM G = 2 takes them all (2,048 chains on 1,024 points: 92 and 178
- * us with G = 1, 79 and 154 with 2), if not for one pass of many chains.
+ * 32 chains per SM G = 2 takes them all (2,048 chains on 1,024 points: 92 and 267
+ * us with G = 1, 80 and 230 with 2), if not for one pass of many chains.
  * One warp per CTA with G = 1, where programs differ in length (random
  * programs on 300 points: 1.70 ms, 1.84 with two warps). */
 cudaError_t launch_loglik_grad(const KParams& p, int sms, double* grad, double* lik, int* later, cudaStream_t st) {

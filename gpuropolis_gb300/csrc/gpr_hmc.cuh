@@ -692,8 +692,10 @@ __device__ __forceinline__ void grad_passes_of(const uint2* prog, int ninstr, in
  * DRAM writes per 44 ms), an instruction is decoded once for G passes, sums
  * and products with a constant or x take their operand where it is, and the
  * constants' shares are reduced together.  65,536 chains of the rational model,
- * 1,024 points, 10 moves of 8 leapfrog steps: 146 -> 82 ms; their gradients
- * alone 1.86 -> 1.0 ms. */
+ * 1,024 points, 10 moves of 8 leapfrog steps: 146 -> 66 ms; their gradients
+ * 2.16 -> 0.98 ms, with the copy to the host.  In mixed populations the warps wait
+ * for instructions (22 of 30 cycles between issues: 8,192 chains with structure
+ * moves on 128 points). */
 template <int MAXR, int G, int NV, bool STREAM>
 __device__ __forceinline__ df eval_loglik_grad(const uint2* prog, int ninstr, int info, const GradSmem& ws,
                                                const DataView& dv, const KParams& p, int lane, int& pts_out, float* g) {

@@ -188,14 +188,17 @@ int gpr_debug_fp_issue(int device, int iters, float* ms_dadd32, float* ms_dadd1,
 int gpr_debug_stage_wait(gpr_handle* h, int polls);
 
 /* Layout autotuner (no reference counterpart): times one block of `steps`
- * MH steps under each valid evaluation layout -- the pipelined kernel (two
+ * MH steps under the layout in force and under each evaluation layout -- the pipelined kernel (two
  * chains per warp) or the lockstep one (one chain per warp), K = 4 or 8
  * points per lane, data held in registers (one pass), read from shared
  * memory in passes or streamed from device memory, transcendental/division
  * ops unrolled or (lockstep kernel) through a compact loop -- then, for the
  * best of those, the CTA size (8 or 4 warps) and, for the lockstep kernel,
  * the CTA barrier period (1, 5 steps, none), on the handle's current state and
- * data; keeps the fastest and restores the state, scores and counters.  Every
+ * data; keeps the fastest (the layout in force unless another is more than 1%
+ * faster) and restores the state, scores and counters.  K = 8 streamed is tried
+ * from half the points on at which it is the default.  For GPR_CONST_HMC handles:
+ * one or two passes per sweep, CTA sizes, staged and streamed.  Every
  * layout gives the same chains bit for bit, so the choice changes speed only.
  * Call after gpr_set_data/gpr_set_state. */
 int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* rolled, float* best_ms);
@@ -204,7 +207,9 @@ int gpr_autotune(gpr_handle* h, int steps, int seed, int* K, int* onepass, int* 
  * on the lockstep kernel.  gpr_set_layout2 also sets the CTA barrier period
  * in MH steps (0 = none) and the warps (chains) per CTA (1, 2, 4 or 8);
  * gpr_set_layout3 also selects the pipelined kernel (pipe = 1: two chains per
- * warp, heavy ops unrolled, the barrier period unused). */
+ * warp, heavy ops unrolled, the barrier period unused).  Three input variables
+ * take passes; with K = 8 (heavy ops unrolled) they are streamed.  Batched data
+ * take K = 4 in passes. */
 int gpr_set_layout(gpr_handle* h, int K, int onepass, int rolled);
 int gpr_set_layout2(gpr_handle* h, int K, int onepass, int rolled, int lockstep, int warps_per_cta);
 int gpr_set_layout3(gpr_handle* h, int K, int onepass, int rolled, int lockstep, int warps_per_cta, int pipe);
@@ -220,8 +225,9 @@ int gpr_layout_streamed(gpr_handle* h);
 
 /* Layout of a GPR_CONST_HMC handle's kernel: warps (chains) per CTA (1, 2, 4
  * or 8) and at most ctas_per_sm resident CTAs per SM (0: as many as fit).
- * Fewer CTAs leave more of each SM's L1 to the gradient tapes; gpr_autotune
- * times a set of these for GPR_CONST_HMC handles. */
+ * gpr_autotune times a set of these for GPR_CONST_HMC handles.  How many passes of
+ * 128 points a sweep takes together follows the data, the chains and the move
+ * schedule (gpr_launch_geometry reports K = 4 or 8 points per lane). */
 int gpr_set_hmc_layout(gpr_handle* h, int warps_per_cta, int ctas_per_sm);
 
 /* Launch geometry chosen for the current dataset: points per lane K, whether
